@@ -16,7 +16,8 @@ SOURCES = ["csrc/speedy_api.cu", "csrc/speedy_noalloc.cu", "csrc/speedy_ensemble
            "csrc/speedy_adjoint.cu", "csrc/held_suarez.cu", "csrc/speedy_selftest.cu"]
 HEADERS = ["csrc/speedy_column.cuh", "csrc/speedy_column_smem.cuh", "csrc/speedy_derived.h",
            "csrc/speedy_kernels.cuh", "csrc/speedy_ensemble.cuh", "csrc/speedy_ad.h",
-           "csrc/speedy_generic.h", "csrc/speedy_vjp.h", "csrc/speedy_pk.cuh",
+           "csrc/speedy_generic.h", "csrc/speedy_vjp.h", "csrc/speedy_vjp_smem.cuh",
+           "csrc/speedy_pk.cuh",
            "../include/speedy_b200.h"]
 OUT = os.path.join(HERE, "libspeedy_b200.so")
 OBJ_DIR = os.path.join(HERE, "_build")
@@ -32,12 +33,11 @@ FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC"]
 # instruction issue, IEEE division and subnormal handling cost several instructions each, and
 # measured against the oracles they change nothing (tendencies, precipitation and diagnostics
 # keep their distances at the printed digits; the only values flushed are transmissivities below
-# 1e-38).  The adjoint keeps IEEE division and subnormals and is compiled without contraction
-# too: its kernel exists in two register budgets (four or two blocks per SM, chosen by the
-# batch's tile count), and only separately rounded arithmetic makes the two give the same bits,
-# so that a member's gradients do not depend on the batch it is served in (with contraction
-# ptxas fused different products in the two; without it the T170 VJP takes 0.566 against
-# 0.529 ms, and the reference's float32 arithmetic rounds every operation as well).
+# 1e-38).  The adjoint keeps subnormals and is compiled without contraction too: the values that
+# decide its branches are rounded like the reference's (its division is fdiv in
+# csrc/speedy_vjp.h, which rounds like the IEEE one), its fused multiply-adds are written out, and
+# its two register budgets give the same bits, so that a member's gradients do not depend on the
+# batch it is served in.
 FORWARD_FLAGS = ["-fmad=false", "-prec-div=false", "-ftz=true"]
 SOURCE_FLAGS = {"csrc/speedy_ensemble.cu": FORWARD_FLAGS,
                 "csrc/speedy_selftest.cu": FORWARD_FLAGS,  # checks the forward's arithmetic

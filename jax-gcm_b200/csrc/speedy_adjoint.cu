@@ -3,127 +3,58 @@
 //
 // Launch 1 is the forward's cloud-top pre-pass over the tile list of speedy_ensemble.cuh (each
 // member's level set S and per-latitude solar table: neither carries a derivative).  Launch 2
-// runs one thread per column, one block per tile: the hand-written reverse pass of speedy_vjp.h
+// runs one thread per column, one warp per block: the reverse pass of speedy_vjp_smem.cuh
 // recomputes the column's forward and walks its terms backwards, writing the state gradients;
-// the 12 parameter gradients are summed per thread, then per block, then added to the tile's
-// member with one atomicAdd per parameter.  A single instance is a one-member plan written
-// into its scratch by a small kernel, so it runs exactly the ensemble's instructions.
+// the 12 parameter gradients are summed per thread, then per warp, then added to the tile's
+// member with one coalesced atomic.  A single instance is a one-member plan written into its
+// scratch by a small kernel, so it runs exactly the ensemble's instructions.
+//
+// Measured (the whole call, against the fully unrolled reverse pass with its arrays in registers
+// and local memory that this replaces): T425 with 16 levels 3,191 -> 1,034 us, T170 with 16
+// levels and verify 578 -> 206 us, T85 with 16 levels 129 -> 57 us.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
 #include <string.h>
 
 #include <algorithm>
+#include <mutex>
 
-#include "speedy_ensemble.cuh"
 #include "speedy_vjp.h"
+
+// the column's first half divides like the rest of the adjoint (speedy_vjp.h, fdiv)
+#define SPD_DIV(a, b) (spdvjp::fdiv((a), (b)))
+#include "speedy_ensemble.cuh"
+#include "speedy_vjp_smem.cuh"
 
 namespace spd {
 
 int check_instance(const spd_desc_t* d, const spd_inputs_t* in, const spd_outputs_t* out);
 Consts make_consts(const spd_desc_t* d, const spd_vgrid_t* vg, const spd_params_t* p);
 
-constexpr int kAdjBlock = 128;
-
-struct VjpArgs {
-  spd_vgrid_t vg;
-  spd_params_t p;
-  uint32_t flags;
-  int model_step, C, il;
-  float ablco2, dt_seconds, q_tend_scale;
-  float qcorv[SPD_MAX_KX], gamlat, pexp;  // orographic correction (SPD_OROGRAPHIC)
-};
-
-// One column's VJP: loads, the reverse pass, stores; adds the parameter gradients to pacc.
-template <int KX>
-__device__ __forceinline__ void vjp_column(const VjpArgs& A, const spd_inputs_t& in,
-                                           const spd_cotangents_t& ct, const spd_grads_t& gr,
-                                           uint32_t Sw, const ZonalRow* __restrict__ table,
-                                           int c, int C, int il, float* pacc) {
-  const spdvjp::Ctx x{&A.vg, &A.p, A.flags, A.model_step, Sw};
-  spdgen::DiffParams<float> g;
-  g.psmin = A.p.psmin; g.trcnv = A.p.trcnv; g.rhil = A.p.rhil; g.rhbl = A.p.rhbl;
-  g.entmax = A.p.entmax; g.smf = A.p.smf; g.trlsc = A.p.trlsc; g.rhlsc = A.p.rhlsc;
-  g.drhlsc = A.p.drhlsc; g.rhblsc = A.p.rhblsc; g.albcl = A.p.albcl; g.albcls = A.p.albcls;
-  spdgen::ColumnIn<float, float> xi;
-  float ct_t[KX], ct_q[KX];
+// Adds the warp's sums of pacc to params, one coalesced atomic.  Sixteen lanes' worth of sums
+// (12 used) are folded by halves: a lane keeps the half of the values its bit selects and adds the
+// other lane's, 16 shuffles where a butterfly per value takes 60.  Every lane must call it.
+__device__ __forceinline__ void warp_add_params(const float* pacc, float* params) {
+  const int lane = threadIdx.x & 31;
+  float v[16];
 #pragma unroll
-  for (int k = 0; k < KX; ++k) {
-    const size_t i = (size_t)k * C + c;
-    xi.t[k] = __ldg(in.temperature + i);
-    xi.q[k] = __ldg(in.specific_humidity + i);
-    xi.phi[k] = __ldg(in.geopotential + i);
-    ct_t[k] = __ldg(ct.temperature + i);
-    ct_q[k] = __ldg(ct.specific_humidity + i);
-  }
-  const size_t lo = (size_t)(KX - 1) * C + c;
-  xi.psa = __ldg(in.normalized_surface_pressure + c);
-  xi.u_low = __ldg(in.u_wind + lo);
-  xi.v_low = __ldg(in.v_wind + lo);
-  xi.sst = __ldg(in.sea_surface_temperature + c);
-  xi.stl = __ldg(in.stl_am + c);
-  xi.soilw = __ldg(in.soilw_am + c);
-  xi.snowc = __ldg(in.snowc_am + c);
-  xi.sice = __ldg(in.sice_am + c);
-  xi.alb0 = __ldg(in.alb0 + c);
-  xi.fmask = __ldg(in.fmask + c);
-  xi.orog = __ldg(in.orog + c);
-  xi.phis0 = __ldg(in.phis0 + c);
-  const ZonalRow z = table[c % il];
-  xi.fsol = z.fsol; xi.ozupp = z.ozupp; xi.ozone = z.ozone; xi.zenit = z.zenit;
-  xi.stratz = z.stratz; xi.sqrt_coa = z.sqrt_coa;
-  spdvjp::Bar<KX, float> b;
-  spdvjp::column_vjp<KX, float>(x, g, A.ablco2, A.dt_seconds, A.q_tend_scale, xi, ct_t, ct_q,
-                                __ldg(ct.u_wind + lo), __ldg(ct.v_wind + lo), b, A.qcorv,
-                                A.gamlat, A.pexp);
+  for (int j = 0; j < 16; ++j) v[j] = j < SPD_NUM_DIFF_PARAMS ? pacc[j] : 0.0f;
 #pragma unroll
-  for (int k = 0; k < KX; ++k) {
-    const size_t i = (size_t)k * C + c;
-    gr.temperature[i] = b.t[k];
-    gr.specific_humidity[i] = b.q[k];
-    gr.geopotential[i] = b.phi[k];
-    gr.u_wind[i] = (k == KX - 1) ? b.u : 0.0f;
-    gr.v_wind[i] = (k == KX - 1) ? b.v : 0.0f;
-  }
-  gr.normalized_surface_pressure[c] = b.psa;
+  for (int n = 8; n >= 1; n /= 2) {
+    const bool hi = (lane & (2 * n)) != 0;
 #pragma unroll
-  for (int j = 0; j < SPD_NUM_DIFF_PARAMS; ++j) pacc[j] += b.par[j];
-}
-
-// Sums pacc over the block and adds it to params with one atomic per parameter.  Every thread
-// of the block must call it.
-__device__ __forceinline__ void block_add_params(float* pacc, float* params) {
-  __shared__ float red[kAdjBlock / 32][SPD_NUM_DIFF_PARAMS];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-  for (int j = 0; j < SPD_NUM_DIFF_PARAMS; ++j) {
-    float v = pacc[j];
-    for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
-    if (lane == 0) red[warp][j] = v;
+    for (int j = 0; j < n; ++j) {
+      const float keep = hi ? v[j + n] : v[j], give = hi ? v[j] : v[j + n];
+      v[j] = keep + __shfl_xor_sync(0xffffffffu, give, 2 * n);
+    }
   }
-  __syncthreads();
-  if (threadIdx.x < SPD_NUM_DIFF_PARAMS) {
-    float v = 0.0f;
-    for (int w = 0; w < kAdjBlock / 32; ++w) v += red[w][threadIdx.x];
-    atomicAdd(params + threadIdx.x, v);
-  }
-  __syncthreads();
+  v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+  const int j = lane >> 1;
+  if ((lane & 1) == 0 && j < SPD_NUM_DIFF_PARAMS) atomicAdd(params + j, v[0]);
 }
 
 // ---- ensemble ----
-struct VjpMemberDev {
-  spd_inputs_t in;
-  spd_cotangents_t ct;
-  spd_grads_t gr;
-  int C, il, kx, cls;
-  uint32_t* S;
-  ZonalRow* table;
-};
-
-struct VjpClassArgs {
-  VjpArgs cls[SPD_MAX_CLASSES];
-};
-
 __global__ void __launch_bounds__(kBlock)
     ensemble_vjp_prepass(const __grid_constant__ ClassArgs A,
                          const VjpMemberDev* __restrict__ members,
@@ -137,36 +68,69 @@ __global__ void __launch_bounds__(kBlock)
   prepass_tiles(A, members, tiles, ntiles);
 }
 
-// Two register budgets of the same kernel: 128 registers for four blocks per SM, or 255 for two
-// (1,376 against 2,088 bytes of stack, ptxas).  Two blocks per SM is the faster where every
-// tile of the batch is resident at once (T85 with 16 levels, 256 tiles: 0.134 against
-// 0.194 ms); four is the faster at T170 (1,024 tiles, 1.73 waves of four-per-SM residency
-// against 3.46 of two).  The launch takes two per SM when the tiles fit in one such wave.  The
-// translation unit is compiled without multiply-add contraction, so the two give the same bits
-// (a member's gradients do not depend on the batch that carried it).
-template <int kMinBlocks>
-__global__ void __launch_bounds__(kAdjBlock, kMinBlocks)
-    ensemble_adjoint(const __grid_constant__ VjpClassArgs A,
+// The adjoint launch: one thread per column (speedy_vjp_smem.cuh), one warp per block with its
+// level arrays in `sm`, so that no warp waits for another and a finished one makes room at once.
+// At 16 levels an arena is 18,432 bytes, which with the 1,024 reserved per block is exactly a
+// twelfth of an SM's shared memory: twelve warps, which 168 registers allow as well.  The threads
+// past a member's last column run that column again and store nothing, so that every warp is whole
+// (the convection's reverse votes).
+// Two register budgets: 168 (three warps per scheduler), or 255 (two), which spills nothing and is
+// the faster where two warps per scheduler hold the whole batch (T85 with 16 levels, 1,024 warps:
+// 60 against 66 us; T170, 4,096 warps: 209 against 194 us).  Both give the same bits, so a
+// member's gradients do not depend on the batch that carried it.
+template <int kWarpsPerSm>
+__global__ void __launch_bounds__(kVjpThreads, kWarpsPerSm)
+    ensemble_adjoint(const __grid_constant__ ClassArgs A,
                      const VjpMemberDev* __restrict__ members, const Tile* __restrict__ tiles,
                      int ntiles) {
-  for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-    const Tile tl = tiles[t];
-    const VjpMemberDev& m = members[tl.member];
-    const int c = tl.col0 + threadIdx.x;
+  constexpr int kPerTile = kNT / kVjpThreads;
+  extern __shared__ float sm[];
+  for (int b = blockIdx.x; b < ntiles * kPerTile; b += gridDim.x) {
+    const Tile tl = tiles[b / kPerTile];
+    const VjpMemberDev* m = members + tl.member;
+    const int C = m->C, col0 = tl.col0 + (b % kPerTile) * kVjpThreads;
+    if (col0 >= C) continue;
+    const bool valid = col0 + (int)threadIdx.x < C;
+    const int c = valid ? col0 + (int)threadIdx.x : C - 1;
     float pacc[SPD_NUM_DIFF_PARAMS];
 #pragma unroll
     for (int j = 0; j < SPD_NUM_DIFF_PARAMS; ++j) pacc[j] = 0.0f;
-    if (c < m.C) {
-      const VjpArgs& V = A.cls[m.cls];
-      const uint32_t Sw = *m.S;
-      switch (m.kx) {  // uniform per block
-        case 16: vjp_column<16>(V, m.in, m.ct, m.gr, Sw, m.table, c, m.C, m.il, pacc); break;
-        case 8: vjp_column<8>(V, m.in, m.ct, m.gr, Sw, m.table, c, m.C, m.il, pacc); break;
-        default: vjp_column<7>(V, m.in, m.ct, m.gr, Sw, m.table, c, m.C, m.il, pacc); break;
-      }
+    const ConstsD& CD = A.cls[m->cls];
+    const uint32_t S = *m->S;
+    const ZonalRow z = m->table[c % m->il];
+    switch (m->kx) {  // uniform per block
+      case 16: column_vjp_smem<16>(CD, sm, m, z, S, c, C, valid, pacc); break;
+      case 8: column_vjp_smem<8>(CD, sm, m, z, S, c, C, valid, pacc); break;
+      default: column_vjp_smem<7>(CD, sm, m, z, S, c, C, valid, pacc); break;
     }
-    block_add_params(pacc, m.gr.params);
+#pragma unroll
+    for (int j = 0; j < SPD_NUM_DIFF_PARAMS; ++j) pacc[j] = valid ? pacc[j] : 0.0f;
+    warp_add_params(pacc, field(&m->gr.params));
   }
+}
+
+// Allows the adjoint launch its arena on the current device, once per device (the attribute is a
+// per-device setting of the kernel); gives the device's SM count.
+static int allow_arena(int* sms = nullptr) {
+  constexpr int kMaxDevices = 64;
+  static std::mutex mu;
+  static int count[kMaxDevices] = {};  // SMs, once set up
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return SPD_ERR_CUDA;
+  std::lock_guard<std::mutex> lock(mu);
+  if (!count[dev]) {
+    const int bytes = (int)vjp_arena_bytes(SPD_MAX_KX);
+    int n = 0;
+    if (cudaFuncSetAttribute(ensemble_adjoint<12>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             bytes) != cudaSuccess ||
+        cudaFuncSetAttribute(ensemble_adjoint<8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             bytes) != cudaSuccess ||
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+      return SPD_ERR_CUDA;
+    count[dev] = n;
+  }
+  if (sms) *sms = count[dev];
+  return SPD_OK;
 }
 
 // The one-member plan of a single instance: its record and its tile list.
@@ -192,14 +156,14 @@ int preload_adjoint() {
   bool ok = true;
   ok &= cudaFuncGetAttributes(&a, vjp_single_plan) == cudaSuccess;
   ok &= cudaFuncGetAttributes(&a, ensemble_vjp_prepass) == cudaSuccess;
-  ok &= cudaFuncGetAttributes(&a, ensemble_adjoint<4>) == cudaSuccess;
-  ok &= cudaFuncGetAttributes(&a, ensemble_adjoint<2>) == cudaSuccess;
-  return ok ? SPD_OK : SPD_ERR_CUDA;
+  ok &= cudaFuncGetAttributes(&a, ensemble_adjoint<12>) == cudaSuccess;
+  ok &= cudaFuncGetAttributes(&a, ensemble_adjoint<8>) == cudaSuccess;
+  return ok && allow_arena() == SPD_OK ? SPD_OK : SPD_ERR_CUDA;
 }
 
 // Both launches over a plan already on the device (tiles at base + tiles_off).
-static int launch_ensemble_vjp(const ClassArgs& P, const VjpClassArgs& V, char* base,
-                               int nmembers, int ntiles, size_t levelset_offset,
+static int launch_ensemble_vjp(const ClassArgs& A, int kx_layout, char* base, int nmembers,
+                               int ntiles, size_t levelset_offset,
                                size_t levelset_bytes, int grid_blocks, cudaStream_t st) {
   const VjpMemberDev* md = reinterpret_cast<const VjpMemberDev*>(base + 256);
   const size_t tiles_off = 256 + align256((size_t)nmembers * sizeof(VjpMemberDev));
@@ -207,39 +171,20 @@ static int launch_ensemble_vjp(const ClassArgs& P, const VjpClassArgs& V, char* 
   // Default: one block per tile.  The blocks are short (one tile's columns each), so the SMs
   // turn over often and a higher-priority stream's kernels (a forward batch) get them within
   // one block's time; a persistent grid would hold every SM until the whole batch is done.
-  const int grid = grid_blocks > 0 ? std::min(grid_blocks, ntiles) : ntiles;
+  const int grid =
+      (grid_blocks > 0 ? std::min(grid_blocks, ntiles) : ntiles) * (kNT / kVjpThreads);
   const int grid_pre = std::min(ntiles, 65535);
+  int sms = 0;
+  if (allow_arena(&sms) != SPD_OK) return SPD_ERR_CUDA;
   if (cudaMemsetAsync(base + levelset_offset, 0, levelset_bytes, st) != cudaSuccess)
     return SPD_ERR_CUDA;
-  int dev = 0, sms = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess ||
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-    return SPD_ERR_CUDA;
-  ensemble_vjp_prepass<<<grid_pre, kBlock, 0, st>>>(P, md, tl, ntiles);
-  if (grid <= 2 * sms)
-    ensemble_adjoint<2><<<grid, kAdjBlock, 0, st>>>(V, md, tl, ntiles);
+  ensemble_vjp_prepass<<<grid_pre, kBlock, 0, st>>>(A, md, tl, ntiles);
+  const size_t arena = vjp_arena_bytes(kx_layout);
+  if (grid <= 8 * sms)
+    ensemble_adjoint<8><<<grid, kVjpThreads, arena, st>>>(A, md, tl, ntiles);
   else
-    ensemble_adjoint<4><<<grid, kAdjBlock, 0, st>>>(V, md, tl, ntiles);
+    ensemble_adjoint<12><<<grid, kVjpThreads, arena, st>>>(A, md, tl, ntiles);
   return cudaGetLastError() == cudaSuccess ? SPD_OK : SPD_ERR_CUDA;
-}
-
-static VjpArgs make_vjp_args(const spd_desc_t* desc, const spd_vgrid_t* vgrid,
-                             const spd_params_t* params) {
-  const Derived D = derive_constants(desc, vgrid, params);
-  VjpArgs A;
-  A.vg = *vgrid;
-  A.p = *params;
-  A.flags = desc->flags;
-  A.model_step = desc->model_step;
-  A.C = desc->ix * desc->il;
-  A.il = desc->il;
-  A.ablco2 = D.ablco2;
-  A.dt_seconds = desc->dt_seconds;
-  A.q_tend_scale = desc->q_tend_scale;
-  for (int k = 0; k < SPD_MAX_KX; ++k) A.qcorv[k] = D.qcorv[k];
-  A.gamlat = D.gamlat;
-  A.pexp = D.pexp;
-  return A;
 }
 
 // The fields spd_vjp reads and writes, validated like spd_fwd's.
@@ -282,11 +227,9 @@ int spd_vjp(const spd_desc_t* desc, const spd_vgrid_t* vgrid, const spd_params_t
   if (desc->kx != 7 && desc->kx != 8 && desc->kx != 16) return SPD_ERR_KX;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   char* base = static_cast<char*>(scratch);
-  ClassArgs P;
-  VjpClassArgs V;
-  P.cls[0].K = make_consts(desc, vgrid, params);
-  P.cls[0].D = derive_constants(desc, vgrid, params);
-  V.cls[0] = make_vjp_args(desc, vgrid, params);
+  ClassArgs A;
+  A.cls[0].K = make_consts(desc, vgrid, params);
+  A.cls[0].D = derive_constants(desc, vgrid, params);
   VjpMemberDev rec;
   rec.in = *in;
   rec.ct = *ct;
@@ -301,7 +244,7 @@ int spd_vjp(const spd_desc_t* desc, const spd_vgrid_t* vgrid, const spd_params_t
   Tile* tiles = reinterpret_cast<Tile*>(base + L.tiles);
   const int grid_init = std::min((L.ntiles + kBlock - 1) / kBlock, 1024);
   vjp_single_plan<<<grid_init, kBlock, 0, st>>>(rec, dst, tiles, L.ntiles);
-  return launch_ensemble_vjp(P, V, base, 1, L.ntiles, L.levelset,
+  return launch_ensemble_vjp(A, desc->kx, base, 1, L.ntiles, L.levelset,
                              align256(sizeof(uint32_t)), 0, st);
 }
 
@@ -356,17 +299,17 @@ int spd_ensemble_vjp(const spd_class_t* classes, int nclasses, void* plan_device
   using namespace spd;
   if (!classes || !plan_device || !info) return SPD_ERR_NULL;
   if (nclasses <= 0 || nclasses > SPD_MAX_CLASSES || info->ntiles <= 0) return SPD_ERR_SHAPE;
-  ClassArgs P;
-  VjpClassArgs V;
+  ClassArgs A;
+  int kx_layout = 0;
   for (int i = 0; i < nclasses; ++i) {
-    P.cls[i].K = make_consts(&classes[i].desc, &classes[i].vgrid, &classes[i].params);
-    P.cls[i].D = derive_constants(&classes[i].desc, &classes[i].vgrid, &classes[i].params);
-    V.cls[i] = make_vjp_args(&classes[i].desc, &classes[i].vgrid, &classes[i].params);
+    A.cls[i].K = make_consts(&classes[i].desc, &classes[i].vgrid, &classes[i].params);
+    A.cls[i].D = derive_constants(&classes[i].desc, &classes[i].vgrid, &classes[i].params);
+    kx_layout = std::max(kx_layout, classes[i].desc.kx);
   }
   // Default: one block per tile.  The blocks are short (one tile's columns each), so the SMs
   // turn over often and a higher-priority stream's kernels (a forward batch) get them within
   // one block's time; a persistent grid would hold every SM until the whole batch is done.
-  return launch_ensemble_vjp(P, V, static_cast<char*>(plan_device), info->nmembers,
+  return launch_ensemble_vjp(A, kx_layout, static_cast<char*>(plan_device), info->nmembers,
                              info->ntiles, info->levelset_offset, info->levelset_bytes,
                              grid_blocks, static_cast<cudaStream_t>(stream));
 }

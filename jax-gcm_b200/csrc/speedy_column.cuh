@@ -12,6 +12,12 @@
 
 #include "speedy_b200.h"
 
+// Division of the parts that the forward and the adjoint share: the translation unit's own, unless
+// it names another (speedy_adjoint.cu).
+#ifndef SPD_DIV
+#define SPD_DIV(a, b) ((a) / (b))
+#endif
+
 namespace spd {
 
 // jcm/constants.py:3-5, physics/speedy/physical_constants.py:9-45
@@ -48,9 +54,9 @@ __device__ __forceinline__ float sq(float x) { return x * x; }
 __device__ __forceinline__ float qsat_of(float ta, float ps, float sig) {
   const float e0 = 6.108e-3f, c1 = 17.269f, c2 = 21.875f, t0 = 273.16f, t1 = 35.86f,
               t2 = 7.66f;
-  float e = (ta >= t0) ? e0 * expf(c1 * (ta - t0) / (ta - t1))
-                       : e0 * expf(c2 * (ta - t0) / (ta - t2));
-  return 622.0f * e / (sig * ps - 0.378f * e);
+  float e = (ta >= t0) ? e0 * expf(SPD_DIV(c1 * (ta - t0), ta - t1))
+                       : e0 * expf(SPD_DIV(c2 * (ta - t0), ta - t2));
+  return SPD_DIV(622.0f * e, sig * ps - 0.378f * e);
 }
 
 // radset (longwave_radiation.py:204-226): band energy fractions times (1 - epslw).
@@ -213,7 +219,7 @@ __device__ __forceinline__ int column_icltop(const Consts& K, const float t[KX],
 #pragma unroll
   for (int k = 0; k < KX; ++k) {
     qsat[k] = qsat_of(t[k], psa, K.vg.fsg[k]);
-    rh[k] = q[k] / qsat[k];
+    rh[k] = SPD_DIV(q[k], qsat[k]);
     se[k] = kCp * t[k] + phi[k];
   }
   float qdif;

@@ -202,9 +202,9 @@ __device__ __forceinline__ void column_first(const ConstsD& C, const float (&T)[
   const Derived& D = C.D;
   const spd_params_t& p = K.p;
   const spd_vgrid_t& vg = K.vg;
-  auto rh_at = [&](int k) { return Q[k] / QS[k]; };  // spec_hum_to_rel_hum (humidity.py:45)
+  auto rh_at = [&](int k) { return SPD_DIV(Q[k], QS[k]); };  // spec_hum_to_rel_hum (humidity.py:45)
   const float psa = s.psa;
-  const float rps = 1.0f / psa;
+  const float rps = SPD_DIV(1.0f, psa);
   float SE[KX];  // dry static energy cp T + phi
 
   // ---- spec_hum_to_rel_hum (humidity.py:16-51) --------------------------------------------
@@ -257,7 +257,7 @@ __device__ __forceinline__ void column_first(const ConstsD& C, const float (&T)[
     const float sb = se_b1 + w_last * (se_b - se_b1);
     const float qb = fminf(q_b1 + w_last * (q_b - q_b1), q_b);
     const float fpsa = psa * fminf(1.0f, (psa - p.psmin) * D.rdps);
-    const float fmass = D.fm0 * fpsa * fminf(5.0f, qdif / (qmax - qb));
+    const float fmass = D.fm0 * fpsa * fminf(5.0f, SPD_DIV(qdif, qmax - qb));
     const float cbmf = mask ? fmass : 0.0f * fmass;
     const float fus = fmass * se_b, fuq = fmass * qmax;
     const float fds = fmass * sb, fdq = fmass * qb;
@@ -388,7 +388,7 @@ __device__ __forceinline__ void column_first(const ConstsD& C, const float (&T)[
       o.icltop = min(iptop, icl);
       return;
     }
-    const float gse = (se_b1 - se_b) / (PHI[KX - 2] - PHI[KX - 1]);
+    const float gse = SPD_DIV(se_b1 - se_b, PHI[KX - 2] - PHI[KX - 1]);
     const float pr1 = fminf(p.pmaxcl, 86.4f * (o.precnv + o.precls));
     cloudc = fminf(1.0f, p.wpcl * sqrtf(fmaxf(kEpsilon, pr1)) + sq(fminf(1.0f, cmax * D.rrcl)));
     if (isnan(cloudc)) cloudc = 1.0f;

@@ -13,9 +13,12 @@
 // max/min/clip ties split the derivative evenly between the two arguments; where() passes it to
 // the chosen branch only; integer level indices (convective top, cloud top, the cloud-top level
 // set) carry none.  The forward arithmetic follows speedy_generic.h operation for operation, so
-// every branch is taken as in the forward kernel that records a tape.
+// every branch is taken as in the host forward that records a tape.
 //
-// The same source builds for the host (F = double or float) and the device (F = float).
+// This file is the adjoint's reference: it builds for the host in double and float, where the tests
+// check it against finite differences and a recorded tape.  The device's column
+// (speedy_vjp_smem.cuh) is the same reverse pass arranged for the chip; it takes the small pieces
+// from here (division, max/min weights, saturation humidity and its partials, the surface fluxes).
 #pragma once
 
 #include <math.h>
@@ -23,21 +26,6 @@
 
 #include "speedy_b200.h"
 #include "speedy_generic.h"
-
-// Loop unrolling on the device: every loop of the reverse pass is unrolled fully (the level
-// count is a template parameter).  Indexed by constants, the small arrays (band fluxes,
-// transmissivities, blackbody fractions and their adjoints) become registers and the per-level
-// arrays are placed by the register allocator, spilled where they must be, instead of all
-// living in local memory behind a dynamic index.  Measured on T170 with 16 levels: 0.916 ms
-// with every loop rolled, 0.777 with the band loops unrolled, level loops unrolled by 2 / 4 / 8
-// 0.748 / 0.728 / 0.701, fully 0.619.
-#if defined(__CUDA_ARCH__)
-#define SPD_BANDS _Pragma("unroll")
-#define SPD_LEVELS _Pragma("unroll")
-#else
-#define SPD_BANDS
-#define SPD_LEVELS
-#endif
 
 namespace spdvjp {
 
@@ -53,6 +41,26 @@ SPD_HD double fsqrt(double x) { return sqrt(x); }
 SPD_HD bool fnan(float x) { return x != x; }
 SPD_HD bool fnan(double x) { return x != x; }
 
+// Division.  On the device: the reciprocal's hardware estimate with one Newton step, then the
+// quotient corrected by its own residual (Markstein), which rounds like the IEEE quotient for
+// operands far from the ends of the exponent range, without the subroutine call of the IEEE one
+// (around which the compiler saves and restores registers).
+#if defined(__CUDA_ARCH__)
+SPD_HD float frcp(float b) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(b));
+  return fmaf(fmaf(-b, r, 1.0f), r, r);
+}
+SPD_HD float fdiv(float a, float b) {
+  const float r = frcp(b), q = a * r;
+  return fmaf(fmaf(-b, q, a), r, q);
+}
+#else
+SPD_HD float frcp(float b) { return 1.0f / b; }
+SPD_HD float fdiv(float a, float b) { return a / b; }
+#endif
+SPD_HD double fdiv(double a, double b) { return a / b; }
+
 // max/min with the value convention of the tape (a tie, NaN included, returns the first).
 template <class F> SPD_HD F vmax(F a, F b) { return a > b ? a : (b > a ? b : a); }
 template <class F> SPD_HD F vmin(F a, F b) { return a < b ? a : (b < a ? b : a); }
@@ -63,7 +71,8 @@ template <class F> SPD_HD F wmin(F a, F b) { return a < b ? F(1) : (b < a ? F(0)
 enum { P_PSMIN, P_TRCNV, P_RHIL, P_RHBL, P_ENTMAX, P_SMF, P_TRLSC, P_RHLSC, P_DRHLSC,
        P_RHBLSC, P_ALBCL, P_ALBCLS, P_N };
 
-// get_qsat (humidity.py:73-104) and its partials with respect to ta and ps.
+// get_qsat (humidity.py:73-104) and its partials with respect to ta and ps.  With q = 622 e / D,
+// D = sig ps - 0.378 e and x = q (1 + (0.378 / 622) q), dq/de = x / e and dq/dps = -x / ps.
 template <class F>
 SPD_HD F qsat_d(F ta, F ps, F sig, F& d_t, F& d_p) {
   const F e0 = F(6.108e-3), t0 = F(273.16);
@@ -71,13 +80,13 @@ SPD_HD F qsat_d(F ta, F ps, F sig, F& d_t, F& d_p) {
   const F c = warm ? F(17.269) : F(21.875);
   const F tt = warm ? F(35.86) : F(7.66);
   const F num = c * (ta - t0), den = ta - tt;
-  const F r = num / den;
+  const F r = fdiv(num, den);
   const F e = e0 * fexp(r);
-  const F de = e * (c / den - r / den);
   const F D = sig * ps - F(0.378) * e;
-  const F q = F(622.0) * e / D;
-  d_t = (F(622.0) / D + (q / D) * F(0.378)) * de;
-  d_p = -(q / D) * sig;
+  const F q = fdiv(F(622.0) * e, D);
+  const F x = q + q * (F(0.378 / 622.0) * q);
+  d_t = x * fdiv(c * (t0 - tt), den * den);  // d ln(e) / dta = c (t0 - tt) / (ta - tt)^2
+  d_p = -fdiv(x, ps);
   return q;
 }
 
@@ -172,7 +181,6 @@ struct Ctx {
 // ---------------------------------------------------------------------------------------------
 template <int KX, class F>
 SPD_HD void humidity(const Ctx& x, Col<KX, F>& c) {
-  SPD_LEVELS
   for (int k = 0; k < KX; ++k) {
     F d_t, d_p;
     c.qsat[k] = qsat_d(c.t[k], c.psa, F(x.vg->fsg[k]), d_t, d_p);
@@ -181,7 +189,6 @@ SPD_HD void humidity(const Ctx& x, Col<KX, F>& c) {
 
 template <int KX, class F>
 SPD_HD void humidity_rev(const Ctx& x, const Col<KX, F>& c, Bar<KX, F>& b) {
-  SPD_LEVELS
   for (int k = 0; k < KX; ++k) {
     F d_t, d_p;
     qsat_d(c.t[k], c.psa, F(x.vg->fsg[k]), d_t, d_p);
@@ -207,7 +214,6 @@ SPD_HD void dconv(const Ctx& x, const DiffParams<F>& g, Col<KX, F>& c) {
   const F mse1 = vmin(mse0, c.SE(KX - 2) + F(2501.0) * c.q[KX - 2]);
   const F mss0 = vmax(mse0, c.SE(KX - 1) + F(2501.0) * c.qsat[KX - 1]);
   int ktop1 = KX, ktop2 = KX;
-  SPD_LEVELS
   for (int k = KX - 4; k >= 2; --k) {
     const F m2 = mss2_at(x, c, k);
     if (mss0 > m2) ktop1 = k + 1;
@@ -234,11 +240,9 @@ SPD_HD void dconv_rev(const Ctx& x, const DiffParams<F>& g, const Col<KX, F>& c,
   const F qthr0 = g.rhbl * c.qsat[KX - 1];
   if (c.case1) {
     const F mse0 = c.SE(KX - 1) + F(2501.0) * c.q[KX - 1];
-    // the threshold level j = ktop2 - 1, matched in a loop so that the per-level arrays are
-    // addressed by constants
+    // the threshold level j = ktop2 - 1, matched in a loop
     const int jt = c.ktop2 - 1;
     F msthr = F(0);
-    SPD_LEVELS
     for (int j = 0; j < KX; ++j)
       if (j == jt) msthr = mss2_at(x, c, j);
     const F A = c.q[KX - 1] - qthr0;
@@ -251,7 +255,6 @@ SPD_HD void dconv_rev(const Ctx& x, const DiffParams<F>& g, const Col<KX, F>& c,
     const F msthr_b = -mse0_b;
     b.add_se(KX - 1, mse0_b);
     b.q[KX - 1] += F(2501.0) * mse0_b;
-    SPD_LEVELS
     for (int j = 0; j < KX - 1; ++j) {
       if (j != jt) continue;
       const F w = F(x.vg->wvi[j][1]);
@@ -285,21 +288,18 @@ SPD_HD void conv(const Ctx& x, const DiffParams<F>& g, const Col<KX, F>& c, Cv<K
   const spd_vgrid_t& vg = *x.vg;
   const int iptop = c.iptop_cv;
   w.sentr = F(0);
-  SPD_LEVELS
   for (int k = 1; k < KX - 1; ++k) {
     const F e = vmax(F(0), F(vg.fsg[k]) - F(0.5));
     w.entr[k] = e * e;
     w.sentr = w.sentr + w.entr[k];
   }
   w.escale = g.entmax / w.sentr;
-  SPD_LEVELS
   for (int k = 1; k < KX - 1; ++k) w.entr[k] = w.entr[k] * w.escale;
   w.fm0 = F(1e5) * F(vg.dhs[KX - 1]) / (F(9.81) * g.trcnv * F(3600.0));
   w.rdps = F(2.0) / (F(1.0) - g.psmin);
   const bool mask = iptop < KX;
   w.qmax = vmax(F(1.01) * c.q[KX - 1], c.qsat[KX - 1]);
   w.sb3[0] = w.qb3[0] = F(0);
-  SPD_LEVELS
   for (int k = 1; k < KX; ++k) {
     w.sb3[k] = c.SE(k - 1) + F(vg.wvi[k - 1][1]) * (c.SE(k) - c.SE(k - 1));
     w.qb3[k] = c.q[k - 1] + F(vg.wvi[k - 1][1]) * (c.q[k] - c.q[k - 1]);
@@ -317,7 +317,6 @@ SPD_HD void conv(const Ctx& x, const DiffParams<F>& g, const Col<KX, F>& c, Cv<K
   w.fds = w.fmass * w.sb;
   w.fdq = w.fmass * w.qb;
   F cm = F(0), cs = F(0), cq = F(0);
-  SPD_LEVELS
   for (int k = KX - 1; k >= 0; --k) {
     const bool lm = (k <= KX - 2) && (k >= iptop);
     F en = (k >= 1 && k <= KX - 2) ? w.entr[k] * c.psa * w.cbmf : F(0);
@@ -333,7 +332,6 @@ SPD_HD void conv(const Ctx& x, const DiffParams<F>& g, const Col<KX, F>& c, Cv<K
   }
   w.dfse[KX - 1] = w.fds - w.fus;
   w.dfqa[KX - 1] = w.fdq - w.fuq;
-  SPD_LEVELS
   for (int k = 0; k < KX - 1; ++k) {
     const bool lm = (k >= iptop);
     const F a = (w.fus3[k + 1] - w.fds3[k + 1]) - (w.fus3[k] - w.fds3[k]);
@@ -342,7 +340,6 @@ SPD_HD void conv(const Ctx& x, const DiffParams<F>& g, const Col<KX, F>& c, Cv<K
     w.dfqa[k] = lm ? bq : F(0) * bq;
   }
   F fsq_sum = F(0);
-  SPD_LEVELS
   for (int k = 0; k < KX; ++k) {
     const bool lm = (k <= KX - 2) && (k >= iptop);
     const F d0 = g.rhil * c.qsat[k] - c.q[k];
@@ -356,7 +353,6 @@ SPD_HD void conv(const Ctx& x, const DiffParams<F>& g, const Col<KX, F>& c, Cv<K
   w.qsatb = w.X = F(0);
   // the top layer k = iptop (1 <= iptop <= kx - 1): a loop over the levels with one match
   // instead of an index, so that the per-level arrays are addressed by constants
-  SPD_LEVELS
   for (int k = 1; k < KX; ++k) {
     if (k != iptop) continue;
     const int kt = k - 1;
@@ -373,7 +369,6 @@ template <int KX, class F>
 SPD_HD void conv_tend(const Ctx& x, const Cv<KX, F>& w, F dt[KX], F dq[KX]) {
   dt[0] = dt[0] + w.dfse[0];
   dq[0] = dq[0] + w.dfqa[0];
-  SPD_LEVELS
   for (int k = 1; k < KX; ++k) {
     dt[k] = dt[k] + w.dfse[k] * w.rps * F(x.vg->grdscp[k]);
     dq[k] = dq[k] + w.dfqa[k] * w.rps * F(x.vg->grdsig[k]);
@@ -389,7 +384,6 @@ SPD_HD F conv_rev(const Ctx& x, const DiffParams<F>& g, const Col<KX, F>& c, Cv<
   F rps_b = F(0);
   dfse_b[0] = dt_b[0];
   dfqa_b[0] = dq_b[0];
-  SPD_LEVELS
   for (int k = 1; k < KX; ++k) {
     dfse_b[k] = dt_b[k] * F(vg.grdscp[k]) * w.rps;
     dfqa_b[k] = dq_b[k] * F(vg.grdsig[k]) * w.rps;
@@ -397,10 +391,8 @@ SPD_HD F conv_rev(const Ctx& x, const DiffParams<F>& g, const Col<KX, F>& c, Cv<
   }
   b.psa += -rps_b * (w.rps / c.psa);
   F fus3_b[KX], fuq3_b[KX], fds3_b[KX], fdq3_b[KX], fm3_b[KX], sb3_b[KX], qb3_b[KX];
-  SPD_LEVELS
   for (int k = 0; k < KX; ++k)
     fus3_b[k] = fuq3_b[k] = fds3_b[k] = fdq3_b[k] = fm3_b[k] = sb3_b[k] = qb3_b[k] = F(0);
-  SPD_LEVELS
   for (int k = 1; k < KX; ++k) {  // the top layer k = iptop, addressed by constants
     if (k != iptop) continue;
     const int kt = k - 1;
@@ -422,7 +414,6 @@ SPD_HD F conv_rev(const Ctx& x, const DiffParams<F>& g, const Col<KX, F>& c, Cv<
   // dfqa[KX-1] -= sum(fsq); dfqa[k] += fsq[k]
   const F fsq_sum_b = -dfqa_b[KX - 1];
   F cbmf_b = F(0);
-  SPD_LEVELS
   for (int k = 0; k < KX; ++k) {
     const bool lm = (k <= KX - 2) && (k >= iptop);
     if (!lm) continue;
@@ -438,7 +429,6 @@ SPD_HD F conv_rev(const Ctx& x, const DiffParams<F>& g, const Col<KX, F>& c, Cv<
   }
   F fds_b = dfse_b[KX - 1], fus_b = -dfse_b[KX - 1];
   F fdq_b = dfqa_b[KX - 1], fuq_b = -dfqa_b[KX - 1];
-  SPD_LEVELS
   for (int k = 0; k < KX - 1; ++k) {
     if (k < iptop) continue;
     const F a = dfse_b[k], q = dfqa_b[k];
@@ -453,7 +443,6 @@ SPD_HD F conv_rev(const Ctx& x, const DiffParams<F>& g, const Col<KX, F>& c, Cv<
   }
   // the downward accumulation of entrainment
   F fmass_b = F(0), CMB = F(0), CSB = F(0), CQB = F(0);
-  SPD_LEVELS
   for (int k = 0; k < KX; ++k) {
     if (k == KX - 1) {
       fds_b += fds3_b[k];
@@ -512,7 +501,6 @@ SPD_HD F conv_rev(const Ctx& x, const DiffParams<F>& g, const Col<KX, F>& c, Cv<
   qb3_b[KX - 1] += qb_b * wmin(w.qb3[KX - 1], c.q[KX - 1]);
   b.q[KX - 1] += qb_b * wmin(c.q[KX - 1], w.qb3[KX - 1]);
   sb3_b[KX - 1] += sb_b;
-  SPD_LEVELS
   for (int k = 1; k < KX; ++k) {
     const F ww = F(vg.wvi[k - 1][1]);
     b.add_se(k - 1, sb3_b[k] - ww * sb3_b[k]);
@@ -542,7 +530,6 @@ SPD_HD void lsc(const Ctx& x, const DiffParams<F>& g, Col<KX, F>& c, F* dt, F* d
   const F psa2 = c.psa * c.psa;
   F psum = F(0);
   int first = 0;
-  SPD_LEVELS
   for (int k = 1; k < KX; ++k) {
     const F sig2 = F(vg.fsg[k]) * F(vg.fsg[k]);
     const F rhref = vmax(g.rhlsc + g.drhlsc * (sig2 - F(1.0)), g.rhblsc);
@@ -574,7 +561,6 @@ SPD_HD void lsc_rev(const Ctx& x, const DiffParams<F>& g, const Col<KX, F>& c, c
   F psum = F(0);
   F rtlsc_b = F(0), psa2_b = F(0);
   // precls = (0 - psum) * psa: psum is needed first
-  SPD_LEVELS
   for (int k = 1; k < KX; ++k) {
     const F sig2 = F(vg.fsg[k]) * F(vg.fsg[k]);
     const F rhref = vmax(g.rhlsc + g.drhlsc * (sig2 - F(1.0)), g.rhblsc);
@@ -583,7 +569,6 @@ SPD_HD void lsc_rev(const Ctx& x, const DiffParams<F>& g, const Col<KX, F>& c, c
   }
   b.psa += precls_b * (F(0) - psum);
   const F psum_b = -precls_b * c.psa;
-  SPD_LEVELS
   for (int k = 1; k < KX; ++k) {
     const F sig2 = F(vg.fsg[k]) * F(vg.fsg[k]);
     const F X = g.rhlsc + g.drhlsc * (sig2 - F(1.0));
@@ -633,7 +618,6 @@ SPD_HD void clouds(const Ctx& x, Col<KX, F>& c, Cl<KX, F>& w, F fmask) {
   const int icl0 = w.m0 ? nl1 : KX;
   w.mk = 0u;
   w.cmax = F(0);
-  SPD_LEVELS
   for (int k = 2; k < KX - 2; ++k) {
     const F drh = c.RH(k) - F(p.rhcl1);
     const bool m = drh > w.cloudc0 && c.q[k] > F(p.qacl);
@@ -643,7 +627,6 @@ SPD_HD void clouds(const Ctx& x, Col<KX, F>& c, Cl<KX, F>& w, F fmask) {
     w.pm[k] = w.cmax;
   }
   int icl = -1;
-  SPD_LEVELS
   for (int k = 2; k < KX - 2; ++k) {
     const int cand = (w.cmax == w.upd[k]) ? (((w.mk >> k) & 1u) ? k : icl0) : icl0;
     icl = cand > icl ? cand : icl;
@@ -712,7 +695,6 @@ SPD_HD void clouds_rev(const Ctx& x, const Col<KX, F>& c, const Cl<KX, F>& w, F 
   const F rrcl = F(1.0) / (F(p.rhcl2) - F(p.rhcl1));
   F cmax_b = cc_b * wmin(w.cmax * rrcl, F(1.0)) * rrcl;
   F cloudc0_b = F(0);
-  SPD_LEVELS
   for (int k = KX - 3; k >= 2; --k) {
     F ub;
     if (k > 2) {
@@ -748,14 +730,12 @@ SPD_HD void shortwave(const Ctx& x, const DiffParams<F>& g, Col<KX, F>& c, const
   const spd_vgrid_t& vg = *x.vg;
   const spd_params_t& p = *x.p;
   const bool cmask = c.icltop < KX;
-  SPD_LEVELS
   for (int k = 0; k < KX; ++k) w.r[k] = (((x.S >> k) & 1u) && cmask) ? g.albcl * c.cloudc : F(0);
   w.r[KX - 1] = g.albcls * c.clstr;
   w.psaz = c.psa * F(z.zenit);
   w.mnq = vmin(F(p.abscl1) * c.qcloud, F(p.abscl2));
   w.acloud = c.cloudc * w.mnq;
   w.tau0[0] = fexp(-w.psaz * F(vg.dhs[0]) * F(p.absdry));
-  SPD_LEVELS
   for (int k = 1; k < KX - 1; ++k) {
     const F abs1 = F(p.absdry) + F(p.absaer) * (F(vg.fsg[k]) * F(vg.fsg[k]));
     const F cl = (k >= c.icltop) ? w.acloud : F(0) * w.acloud;
@@ -766,7 +746,6 @@ SPD_HD void shortwave(const Ctx& x, const DiffParams<F>& g, Col<KX, F>& c, const
     w.tau0[KX - 1] = fexp(-w.psaz * F(vg.dhs[KX - 1]) * (abs1 + F(p.abswv1) * c.q[KX - 1]));
   }
   w.tau1[0] = F(1);
-  SPD_LEVELS
   for (int k = 1; k < KX; ++k)
     w.tau1[k] = fexp(-w.psaz * F(vg.dhs[k]) * F(p.abswv2) * c.q[k]);
   F f1 = F(z.fsol) * F(0.95);
@@ -781,7 +760,6 @@ SPD_HD void shortwave(const Ctx& x, const DiffParams<F>& g, Col<KX, F>& c, const
   F rs[KX];
   rs[0] = w.r[0];
   rs[1] = w.r[1];
-  SPD_LEVELS
   for (int k = 2; k < KX; ++k) {
     const F prev = f1;
     w.f1v[k] = prev;
@@ -791,7 +769,6 @@ SPD_HD void shortwave(const Ctx& x, const DiffParams<F>& g, Col<KX, F>& c, const
   }
   w.f1 = f1;
   F f2 = F(z.fsol) * F(0.05);
-  SPD_LEVELS
   for (int k = 1; k < KX; ++k) {
     const F prev = f2;
     w.f2v[k] = prev;
@@ -802,7 +779,6 @@ SPD_HD void shortwave(const Ctx& x, const DiffParams<F>& g, Col<KX, F>& c, const
   F up = f1 * c.albsfc;
   w.upv[KX] = up;
   w.dfabs[KX - 1] = w.dfabs[KX - 1] + up * (F(1) - w.tau0[KX - 1]);
-  SPD_LEVELS
   for (int k = KX - 1; k >= 1; --k) {
     up = up * w.tau0[k] + rs[k];
     w.upv[k] = up;
@@ -821,7 +797,6 @@ SPD_HD void shortwave_rev(const Ctx& x, const DiffParams<F>& g, const Col<KX, F>
   const spd_params_t& p = *x.p;
   const bool swon = (x.model_step % 3) == 0;
   F dfabs_b[KX], tau0_b[KX], tau1_b[KX], r_b[KX], rs_b[KX];
-  SPD_LEVELS
   for (int k = 0; k < KX; ++k) {
     dfabs_b[k] = F(0);
     if (swon) {
@@ -836,7 +811,6 @@ SPD_HD void shortwave_rev(const Ctx& x, const DiffParams<F>& g, const Col<KX, F>
   tau0_b[0] += fsw0_b * w.upv[1];
   F up_b = fsw0_b * w.tau0[0];
   r_b[0] += fsw0_b;
-  SPD_LEVELS
   for (int k = 1; k < KX; ++k) {
     up_b += dfabs_b[k - 1] * (F(1) - w.tau0[k - 1]);
     tau0_b[k - 1] -= dfabs_b[k - 1] * w.upv[k];
@@ -847,14 +821,12 @@ SPD_HD void shortwave_rev(const Ctx& x, const DiffParams<F>& g, const Col<KX, F>
   up_b += dfabs_b[KX - 1] * (F(1) - w.tau0[KX - 1]);
   tau0_b[KX - 1] -= dfabs_b[KX - 1] * w.upv[KX];
   f1_b += up_b * c.albsfc;
-  SPD_LEVELS
   for (int k = KX - 1; k >= 1; --k) {
     tau1_b[k] += f2_b * w.f2v[k] - dfabs_b[k] * w.f2v[k];
     f2_b = f2_b * w.tau1[k] + dfabs_b[k] * (F(1) - w.tau1[k]);
   }
   r_b[1] += rs_b[1];
   r_b[0] += rs_b[0];
-  SPD_LEVELS
   for (int k = KX - 1; k >= 2; --k) {
     const F prev = w.f1v[k];
     const F om = F(1) - w.r[k];
@@ -878,7 +850,6 @@ SPD_HD void shortwave_rev(const Ctx& x, const DiffParams<F>& g, const Col<KX, F>
     b.psa -= fa_b * w.tau0[0] * F(z.ozupp);
   }
   F psaz_b = F(0), acloud_b = F(0);
-  SPD_LEVELS
   for (int k = 1; k < KX; ++k) {
     const F Eb = tau1_b[k] * w.tau1[k];
     const F c0 = F(vg.dhs[k]) * F(p.abswv2);
@@ -886,7 +857,6 @@ SPD_HD void shortwave_rev(const Ctx& x, const DiffParams<F>& g, const Col<KX, F>
     psaz_b += -Eb * c0 * c.q[k];
   }
   psaz_b += -tau0_b[0] * w.tau0[0] * F(vg.dhs[0]) * F(p.absdry);
-  SPD_LEVELS
   for (int k = 1; k < KX; ++k) {
     const F Eb = tau0_b[k] * w.tau0[k];
     const F abs1 = F(p.absdry) + F(p.absaer) * (F(vg.fsg[k]) * F(vg.fsg[k]));
@@ -903,7 +873,6 @@ SPD_HD void shortwave_rev(const Ctx& x, const DiffParams<F>& g, const Col<KX, F>
   b.par[P_ALBCLS] += r_b[KX - 1] * c.clstr;
   clstr_b += r_b[KX - 1] * g.albcls;
   const bool cmask = c.icltop < KX;
-  SPD_LEVELS
   for (int k = 0; k < KX - 1; ++k) {
     if (((x.S >> k) & 1u) && cmask) {
       b.par[P_ALBCL] += r_b[k] * c.cloudc;
@@ -956,7 +925,6 @@ SPD_HD void lw_level(const Ctx& x, const Col<KX, F>& c, int k, F ablco2, LwLevel
   F a[4];
   lw_absorb(x, c, k, ablco2, a);
   const F dh = F(x.vg->dhs[k]);
-  SPD_BANDS
   for (int b = 0; b < 4; ++b) L.tau[b] = fexp(-a[b] * c.psa * dh);
   const F sbc = F(5.67e-8);
   if (k == 0) {
@@ -983,7 +951,6 @@ SPD_HD void longwave_down(const Ctx& x, Col<KX, F>& c, F ablco2, Lw<KX, F>& w) {
   LwLevel<F> L;
   lw_level(x, c, 0, ablco2, L);
   radset_d(c.t[0], F(p.epslw), fb, dfb);
-  SPD_BANDS
   for (int b = 0; b < 4; ++b) {
     const F emis = F(1) - L.tau[b];
     w.fld[0][b] = emis * (fb[b] * (L.st0 + emis * L.st1));
@@ -992,11 +959,9 @@ SPD_HD void longwave_down(const Ctx& x, Col<KX, F>& c, F ablco2, Lw<KX, F>& w) {
   F sprev = ((w.fld[0][0] + w.fld[0][1]) + w.fld[0][2]) + w.fld[0][3];
   c.dfl[0] = F(0) + (-sprev);
   F st0_last = L.st0;
-  SPD_LEVELS
   for (int k = 1; k < KX; ++k) {
     lw_level(x, c, k, ablco2, L);
     radset_d(c.t[k], F(p.epslw), fb, dfb);
-    SPD_BANDS
     for (int b = 0; b < 4; ++b) {
       const F emis = F(1) - L.tau[b];
       w.fld[k][b] = L.tau[b] * w.fld[k - 1][b] + emis * (fb[b] * (L.st0 + emis * L.st1));
@@ -1024,15 +989,12 @@ SPD_HD void longwave_up(const Ctx& x, Col<KX, F>& c, const SurfaceRow& z, F ablc
   LwLevel<F> L;
   radset_d(c.tsfc, F(p.epslw), fb, dfb);
   const F fsw[4] = {c.fsw0, c.fsw1, F(0), F(0)};
-  SPD_BANDS
   for (int b = 0; b < 4; ++b) w.flu[KX][b] = fb[b] * c.rlus2 + refsfc * fsw[b];
   c.dfl[KX - 1] = c.dfl[KX - 1] + F(p.epslw) * c.rlus2;
   F sk = ((w.flu[KX][0] + w.flu[KX][1]) + w.flu[KX][2]) + w.flu[KX][3];
-  SPD_LEVELS
   for (int k = KX - 1; k >= 1; --k) {
     lw_level(x, c, k, ablco2, L);
     radset_d(c.t[k], F(p.epslw), fb, dfb);
-    SPD_BANDS
     for (int b = 0; b < 4; ++b) {
       const F emis = F(1) - L.tau[b];
       w.flu[k][b] = L.tau[b] * w.flu[k + 1][b] + emis * (fb[b] * (L.st0 - emis * L.st1));
@@ -1044,7 +1006,6 @@ SPD_HD void longwave_up(const Ctx& x, Col<KX, F>& c, const SurfaceRow& z, F ablc
   lw_level(x, c, 0, ablco2, L);
   radset_d(c.t[0], F(p.epslw), fb, dfb);
   F top[2];
-  SPD_BANDS
   for (int b = 0; b < 2; ++b) {
     const F emis = F(1) - L.tau[b];
     top[b] = L.tau[b] * w.flu[1][b] + emis * (fb[b] * (L.st0 - emis * L.st1));
@@ -1090,7 +1051,6 @@ SPD_HD void lw_level_rev(const Ctx& x, const Col<KX, F>& c, int k, F ablco2,
   lw_absorb(x, c, k, ablco2, a);
   const F dh = F(x.vg->dhs[k]);
   F ab[4];
-  SPD_BANDS
   for (int bb = 0; bb < 4; ++bb) {
     const F Eb = tau_b[bb] * L.tau[bb];
     ab[bb] = -Eb * c.psa * dh;
@@ -1156,7 +1116,6 @@ SPD_HD void longwave_rev_up(const Ctx& x, const Col<KX, F>& c, const SurfaceRow&
   const spd_vgrid_t& vg = *x.vg;
   const spd_params_t& p = *x.p;
   auto dflb = [&](int k) { return dt_b[k] * F(vg.grdscp[k]) / c.psa; };
-  SPD_LEVELS
   for (int k = 0; k < KX; ++k) b.psa += -dt_b[k] * ((c.dfl[k] * F(vg.grdscp[k])) / c.psa) / c.psa;
   F st0b_0, st0b_1;
   {
@@ -1179,7 +1138,6 @@ SPD_HD void longwave_rev_up(const Ctx& x, const Col<KX, F>& c, const SurfaceRow&
     radset_d(c.t[0], F(p.epslw), fb, dfb);
     F tb[4] = {F(0), F(0), F(0), F(0)};
     F s0b = st0b_0, s1b = F(0);
-    SPD_BANDS
     for (int bb = 0; bb < 2; ++bb) {
       F ub_prev;
       lw_step_rev(-dflb(0), L.tau[bb], w.flu[1][bb], fb[bb], dfb[bb], L.st0, L.st1, F(-1),
@@ -1188,14 +1146,12 @@ SPD_HD void longwave_rev_up(const Ctx& x, const Col<KX, F>& c, const SurfaceRow&
     }
     lw_level_rev(x, c, 0, ablco2, L, tb, s0b, s1b, acl1_b, acl2_b, b);
   }
-  SPD_LEVELS
   for (int k = 1; k < KX; ++k) {
     const F Sb = (k >= 2 ? dflb(k - 1) : F(0)) - dflb(k);
     lw_level(x, c, k, ablco2, L);
     radset_d(c.t[k], F(p.epslw), fb, dfb);
     F tb[4] = {F(0), F(0), F(0), F(0)};
     F s0b = (k == 1) ? st0b_1 : F(0), s1b = F(0);
-    SPD_BANDS
     for (int bb = 0; bb < 4; ++bb) {
       F nb;
       lw_step_rev(Ub[bb] + Sb, L.tau[bb], w.flu[k + 1][bb], fb[bb], dfb[bb], L.st0, L.st1,
@@ -1208,7 +1164,6 @@ SPD_HD void longwave_rev_up(const Ctx& x, const Col<KX, F>& c, const SurfaceRow&
   F fbs[4], dfbs[4];
   radset_d(c.tsfc, F(p.epslw), fbs, dfbs);
   rlus2_b = dflb(KX - 1) * F(p.epslw);
-  SPD_BANDS
   for (int bb = 0; bb < 4; ++bb) {
     const F u = Ub[bb] + dflb(KX - 1);
     rlus2_b += u * fbs[bb];
@@ -1227,11 +1182,9 @@ SPD_HD void longwave_rev_down(const Ctx& x, const Col<KX, F>& c, const Lw<KX, F>
   auto dflb = [&](int k) { return dt_b[k] * F(vg.grdscp[k]) / c.psa; };
   const F corlw_b = rlds_b - dflb(KX - 1);
   F Db[4];
-  SPD_BANDS
   for (int bb = 0; bb < 4; ++bb) Db[bb] = rlds_b * F(p.emisfc);
   F fb[4], dfb[4];
   LwLevel<F> L;
-  SPD_LEVELS
   for (int k = KX - 1; k >= 0; --k) {
     const F Sb = -dflb(k) + (k < KX - 1 ? dflb(k + 1) : F(0));
     lw_level(x, c, k, ablco2, L);
@@ -1239,7 +1192,6 @@ SPD_HD void longwave_rev_down(const Ctx& x, const Col<KX, F>& c, const Lw<KX, F>
     F tb[4] = {F(0), F(0), F(0), F(0)};
     F s0b = (k == KX - 1) ? corlw_b * (F(p.epslw) * F(p.emisfc)) : F(0), s1b = F(0);
     const int nb_ = (k == 0) ? 2 : 4;
-    SPD_BANDS
     for (int bb = 0; bb < 4; ++bb) {
       if (bb >= nb_) continue;
       F nb;
@@ -1281,19 +1233,19 @@ SPD_HD void surface(const Ctx& x, Col<KX, F>& c, const SurfaceIn& s, const Surfa
   w.u0 = F(p.fwind0) * c.u;
   w.v0 = F(p.fwind0) * c.v;
   const F astab = (x.flags & SPD_LSCASYM) ? F(0.5) : F(1.0);
-  const F rdth = F(p.fstab) / F(p.dtheta);
+  const F rdth = fdiv(F(p.fstab), F(p.dtheta));
   const bool land = (x.flags & SPD_LFLUXLAND) != 0;
   w.ustr0 = w.ustr1 = w.vstr0 = w.vstr1 = w.shf0 = w.evap0 = w.rlus0 = F(0);
   w.t1_1 = w.q1_1 = w.denv2 = F(0);
   c.rlus2 = F(0);
   c.tsfc = F(0);
   w.ustr2 = w.vstr2 = w.shf2 = w.evap2 = F(0);
-  w.rps = F(1) / c.psa;
+  w.rps = fdiv(F(1), c.psa);
   if (!land) return;
   const F rcp = F(1.0 / 1004.0);
   w.dt1 = F(vg.wvi[KX - 1][1]) * (ta1 - ta2);
   w.t1_0p = F(0) + (ta1 + w.dt1);
-  w.t1_1p = w.t1_0p - phi0 * w.dt1 / (F(2.0 / 7.0 * 1004.0 * 288.0) * F(vg.sigl[KX - 1]));
+  w.t1_1p = w.t1_0p - fdiv(phi0 * w.dt1, F(2.0 / 7.0 * 1004.0 * 288.0) * F(vg.sigl[KX - 1]));
   w.t2_1 = ta1 + rcp * c.phi[KX - 1];
   w.t2_0 = w.t2_1 - rcp * phi0;
   w.warm = ta1 > ta2;
@@ -1305,7 +1257,7 @@ SPD_HD void surface(const Ctx& x, Col<KX, F>& c, const SurfaceIn& s, const Surfa
     w.t1_1 = ta1;
   }
   w.t0 = w.t1_1 + F(s.fmask) * (w.t1_0 - w.t1_1);
-  w.A = F(1e5) * c.psa / (F(2.0 / 7.0 * 1004.0) * w.t0);
+  w.A = fdiv(F(1e5) * c.psa, F(2.0 / 7.0 * 1004.0) * w.t0);
   w.B = fsqrt(w.u0 * w.u0 + w.v0 * w.v0 + F(p.vgust) * F(p.vgust));
   w.denv0 = w.A * w.B;
   const F kts = F(p.ctday) * F(z.sqrt_coa);
@@ -1314,7 +1266,7 @@ SPD_HD void surface(const Ctx& x, Col<KX, F>& c, const SurfaceIn& s, const Surfa
   w.dthl_v = w.tsk_gt ? vmin(F(p.dtheta), w.tskin - w.t2_0)
                       : vmax(-F(p.dtheta), astab * (w.tskin - w.t2_0));
   w.denv1 = w.denv0 * (F(1) + w.dthl_v * rdth);
-  const F rhdrag = F(1) / (F(9.81) * F(p.hdrag));
+  const F rhdrag = fdiv(F(1), F(9.81) * F(p.hdrag));
   const F ph = F(s.phis0) > F(0) ? F(s.phis0) : F(0);
   w.forog = F(1) + rhdrag * (F(1) - fexp(-ph * rhdrag));
   w.cdldv = F(p.cdl) * w.denv0 * w.forog;
@@ -1323,7 +1275,7 @@ SPD_HD void surface(const Ctx& x, Col<KX, F>& c, const SurfaceIn& s, const Surfa
   const F chlcp = F(p.chl) * F(1004.0);
   w.shf0 = chlcp * w.denv1 * (w.tskin - w.t1_0);
   const bool fh = F(p.fhum0) > F(0);
-  w.qs10 = qsat_d(w.t1_0, c.psa, F(1), w.qs10_t, w.qs10_p);
+  if (fh) w.qs10 = qsat_d(w.t1_0, c.psa, F(1), w.qs10_t, w.qs10_p);
   w.q1_0 = fh ? F(p.fhum0) * (c.RH(KX - 1) * w.qs10) + (F(1) - F(p.fhum0)) * c.q[KX - 1]
               : c.q[KX - 1];
   w.qs00 = qsat_d(w.tskin, c.psa, F(1), w.qs00_t, w.qs00_p);
@@ -1342,7 +1294,7 @@ SPD_HD void surface(const Ctx& x, Col<KX, F>& c, const SurfaceIn& s, const Surfa
     w.evap_pos = w.evap0 > F(0);
     w.qs01 = w.evap_pos ? F(s.soilw) * (w.qs01r - w.qs00) : F(0);
     w.den = clamb + w.drls + (F(p.chl) * w.denv1 * (F(1004.0) + (F(2501.0) * w.qs01)));
-    w.dtskin = w.hfl0 / w.den;
+    w.dtskin = fdiv(w.hfl0, w.den);
     w.shf0 = w.shf0 + chlcp * w.denv1 * w.dtskin;
     w.evap0 = w.evap0 + F(p.chl) * w.denv1 * w.qs01 * w.dtskin;
     w.rlus0 = w.rlus0 + w.drls * w.dtskin;
@@ -1351,7 +1303,7 @@ SPD_HD void surface(const Ctx& x, Col<KX, F>& c, const SurfaceIn& s, const Surfa
   w.dths_v = w.sst_gt ? vmin(F(p.dtheta), F(s.sst) - w.t2_1)
                       : vmax(-F(p.dtheta), astab * (F(s.sst) - w.t2_1));
   w.denv2 = w.denv0 * (F(1) + w.dths_v * rdth);
-  w.qs11 = qsat_d(w.t1_1, c.psa, F(1), w.qs11_t, w.qs11_p);
+  if (fh) w.qs11 = qsat_d(w.t1_1, c.psa, F(1), w.qs11_t, w.qs11_p);
   w.q1_1 = fh ? F(p.fhum0) * (c.RH(KX - 1) * w.qs11) + (F(1) - F(p.fhum0)) * c.q[KX - 1]
               : c.q[KX - 1];
   w.cdsdv = F(p.cds) * w.denv2;
@@ -1388,12 +1340,12 @@ SPD_HD void surface_rev(const Ctx& x, const Col<KX, F>& c, const SurfaceIn& s,
   if (!(x.flags & SPD_LFLUXLAND)) return;  // every flux is a constant zero
   const F esbc = F(p.emisfc) * F(5.67e-8);
   const F astab = (x.flags & SPD_LSCASYM) ? F(0.5) : F(1.0);
-  const F rdth = F(p.fstab) / F(p.dtheta);
+  const F rdth = fdiv(F(p.fstab), F(p.dtheta));
   const F chlcp = F(p.chl) * F(1004.0);
   const F gs = F(vg.grdsig[KX - 1]), gc = F(vg.grdscp[KX - 1]);
   const F rps_b = du_b * w.ustr2 * gs + dv_b * w.vstr2 * gs + dtK_b * w.shf2 * gc +
                   dqK_b * w.evap2 * gs;
-  b.psa += -rps_b * (w.rps / c.psa);
+  b.psa += -rps_b * (w.rps * w.rps);
   const F ustr2_b = du_b * gs * w.rps, vstr2_b = dv_b * gs * w.rps;
   const F shf2_b = dtK_b * gc * w.rps, evap2_b = dqK_b * gs * w.rps;
   const F fm = F(s.fmask);
@@ -1448,8 +1400,8 @@ SPD_HD void surface_rev(const Ctx& x, const Col<KX, F>& c, const SurfaceIn& s,
     denv1_b += shf0_b * chlcp * w.dtskin + evap0_b * F(p.chl) * w.qs01 * w.dtskin;
     F qs01_b = evap0_b * F(p.chl) * w.denv1 * w.dtskin;
     drls_b += rlus0_b * w.dtskin;
-    const F hfl0_b = dtskin_b / w.den;
-    const F den_b = -dtskin_b * (w.dtskin / w.den);
+    const F hfl0_b = fdiv(dtskin_b, w.den);
+    const F den_b = -hfl0_b * w.dtskin;
     drls_b += den_b;
     denv1_b += den_b * F(p.chl) * (F(1004.0) + F(2501.0) * w.qs01);
     qs01_b += den_b * F(p.chl) * w.denv1 * F(2501.0);
@@ -1522,12 +1474,13 @@ SPD_HD void surface_rev(const Ctx& x, const Col<KX, F>& c, const SurfaceIn& s,
   // denv0 = A B
   {
     const F A_b = denv0_b * w.B, B_b = denv0_b * w.A;
-    const F Bs_b = B_b * (F(0.5) / w.B);
+    const F Bs_b = fdiv(B_b * F(0.5), w.B);
     ua_b += Bs_b * F(2) * w.u0 * F(p.fwind0);
     va_b += Bs_b * F(2) * w.v0 * F(p.fwind0);
     const F K2 = F(2.0 / 7.0 * 1004.0);
-    b.psa += A_b * F(1e5) / (K2 * w.t0);
-    const F t0_b = -A_b * (w.A / w.t0);
+    const F At = fdiv(A_b, w.t0);
+    b.psa += At * (F(1e5) / K2);
+    const F t0_b = -At * w.A;
     t1_1_b += t0_b - F(s.fmask) * t0_b;
     t1_0_b += t0_b * F(s.fmask);
   }
@@ -1546,7 +1499,7 @@ SPD_HD void surface_rev(const Ctx& x, const Col<KX, F>& c, const SurfaceIn& s,
   b.phi[KX - 1] += t2_1_b * rcp;
   const F phi0 = F(s.orog) * F(9.81);
   t1_0p_b += t1_1p_b;
-  F dt1_b = -t1_1p_b * phi0 / (F(2.0 / 7.0 * 1004.0 * 288.0) * F(vg.sigl[KX - 1]));
+  F dt1_b = -fdiv(t1_1p_b * phi0, F(2.0 / 7.0 * 1004.0 * 288.0) * F(vg.sigl[KX - 1]));
   ta1_b += t1_0p_b;
   dt1_b += t1_0p_b;
   const F ww = F(vg.wvi[KX - 1][1]);
@@ -1591,7 +1544,6 @@ SPD_HD void vdiff(const Ctx& x, const Col<KX, F>& c, F* dt, F* dq) {
   const int nl1 = KX - 1;
   const int icnv = KX - c.iptop - 1;
   F tt[KX], qt[KX];
-  SPD_LEVELS
   for (int k = 0; k < KX; ++k) tt[k] = qt[k] = F(0);
   const F dmse = c.SE(KX - 1) - c.SE(nl1 - 1) + F(2501.0) * (c.q[KX - 1] - c.qsat[nl1 - 1]);
   const F drh = c.RH(KX - 1) - c.RH(nl1 - 1);
@@ -1611,7 +1563,6 @@ SPD_HD void vdiff(const Ctx& x, const Col<KX, F>& c, F* dt, F* dq) {
     qt[KX - 1] = -fq * (F(1) / F(vg.dhs[KX - 1]));
   }
   F fluxq[KX];
-  SPD_LEVELS
   for (int k = 2; k < KX - 2; ++k) {
     const bool cond = F(vg.hsg[k + 1]) > F(0.5);
     const F d0 = F(p.rhgrad) * (F(vg.fsg[k + 1]) - F(vg.fsg[k]));
@@ -1620,22 +1571,18 @@ SPD_HD void vdiff(const Ctx& x, const Col<KX, F>& c, F* dt, F* dq) {
     fluxq[k] = (dr >= d0 && cond) ? f2 * c.qsat[k] * dr : F(0);
     qt[k] = qt[k] + fluxq[k] * (F(1) / F(vg.dhs[k]));
   }
-  SPD_LEVELS
   for (int k = 2; k < KX - 2; ++k) qt[k + 1] = qt[k + 1] + (-fluxq[k] * (F(1) / F(vg.dhs[k + 1])));
   F fse[KX];
-  SPD_LEVELS
   for (int k = 0; k < nl1; ++k) {
     const F se0 = c.SE(k + 1) - F(p.segrad) * (c.phi[k + 1] - c.phi[k]);
     fse[k] = (c.SE(k) < se0) ? v.fvdise * (se0 - c.SE(k)) : F(0);
     tt[k] = tt[k] + fse[k] * (F(1) / F(vg.dhs[k]));
   }
   F cum = F(0);
-  SPD_LEVELS
   for (int k = 0; k < nl1; ++k) {
     cum = cum + fse[k] * (F(1) / (F(1) - F(vg.hsg[k + 1])));
     tt[k + 1] = tt[k + 1] + (-cum);
   }
-  SPD_LEVELS
   for (int k = 0; k < KX; ++k) {
     dt[k] = dt[k] + tt[k];
     dq[k] = dq[k] + qt[k];
@@ -1652,7 +1599,6 @@ SPD_HD void vdiff_rev(const Ctx& x, const Col<KX, F>& c, const F* dt_b, const F*
   const int icnv = KX - c.iptop - 1;
   // the cumulative flux: tt[k+1] -= sum_{j<=k} fse[j] / (1 - hsg[j+1])
   F acc = F(0);
-  SPD_LEVELS
   for (int k = nl1 - 1; k >= 0; --k) {
     acc += -dt_b[k + 1];
     const F fse_b = acc * (F(1) / (F(1) - F(vg.hsg[k + 1]))) + dt_b[k] * (F(1) / F(vg.dhs[k]));
@@ -1665,7 +1611,6 @@ SPD_HD void vdiff_rev(const Ctx& x, const Col<KX, F>& c, const F* dt_b, const F*
       b.phi[k] += s_b * F(p.segrad);
     }
   }
-  SPD_LEVELS
   for (int k = 2; k < KX - 2; ++k) {
     const bool cond = F(vg.hsg[k + 1]) > F(0.5);
     const F d0 = F(p.rhgrad) * (F(vg.fsg[k + 1]) - F(vg.fsg[k]));
@@ -1722,7 +1667,6 @@ SPD_HD void column_vjp(const Ctx& x, const DiffParams<F>& g, F ablco2, F dt_seco
   const spd_params_t& p = *x.p;
   const bool verify = (x.flags & SPD_FUSE_VERIFY) != 0;
   Col<KX, F> c;
-  SPD_LEVELS
   for (int k = 0; k < KX; ++k) {
     c.t[k] = in.t[k];
     c.q[k] = (verify && in.q[k] < F(0)) ? F(0) : in.q[k];
@@ -1745,7 +1689,6 @@ SPD_HD void column_vjp(const Ctx& x, const DiffParams<F>& g, F ablco2, F dt_seco
   }
   // ---- forward ----
   F dq[KX], dt[KX];
-  SPD_LEVELS
   for (int k = 0; k < KX; ++k) dq[k] = dt[k] = F(0);
   humidity(x, c);
   dconv(x, g, c);
@@ -1780,11 +1723,9 @@ SPD_HD void column_vjp(const Ctx& x, const DiffParams<F>& g, F ablco2, F dt_seco
     vdiff(x, c, dt, dq);
     if (qcorv && (x.flags & SPD_OROGRAPHIC)) {  // the last term's humidity tendency
       const F qcorh = orographic_qcorh(in.phis0, in.fmask, in.stl, in.sst, F(gamlat), F(pexp));
-      SPD_LEVELS
       for (int k = 0; k < KX; ++k) dq[k] = dq[k] + (qcorh * F(qcorv[k])) / dt_seconds;
     }
   }
-  SPD_LEVELS
   for (int k = 0; k < KX; ++k) {
     F qb = ct_q[k] * q_tend_scale;
     if (verify && !(in.q[k] + dt_seconds * dq[k] >= F(0))) {
@@ -1793,11 +1734,9 @@ SPD_HD void column_vjp(const Ctx& x, const DiffParams<F>& g, F ablco2, F dt_seco
     }
     dq_b[k] = qb;
   }
-  SPD_LEVELS
   for (int k = 0; k < KX; ++k)
     b.t[k] = b.q[k] = b.phi[k] = b.qsat[k] = F(0);
   b.psa = b.u = b.v = F(0);
-  SPD_BANDS
   for (int j = 0; j < P_N; ++j) b.par[j] = F(0);
   // ---- reverse ----
   vdiff_rev(x, c, dt_b, dq_b, b);
@@ -1822,7 +1761,6 @@ SPD_HD void column_vjp(const Ctx& x, const DiffParams<F>& g, F ablco2, F dt_seco
   const F qdif_b = conv_rev(x, g, c, sc.cv, dt_b, dq_b, precnv_b, b);
   dconv_rev(x, g, c, qdif_b, b);
   humidity_rev(x, c, b);
-  SPD_LEVELS
   for (int k = 0; k < KX; ++k) {
     const F qb = (verify && in.q[k] < F(0)) ? F(0) : b.q[k];
     b.q[k] = qb + (((limited >> k) & 1u) ? -(ct_q[k] * q_tend_scale) / dt_seconds : F(0));
