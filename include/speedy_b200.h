@@ -153,12 +153,12 @@ typedef struct {
 size_t spd_fwd_scratch_bytes(const spd_desc_t* desc);
 
 /* SpeedyPhysics.compute_tendencies for one instance (speedy_physics.py:88-127).
- * Two launches on `stream`, each over every column: a light one that forms the instance's
- * cloud-top level set (shortwave_radiation.py:62-68: the cloud tops of every column, from
- * humidity, convection, condensation and clouds) and its per-latitude solar table; then every
- * column whole in one pass (all terms, verify_tendencies when on, every output).  They are the
- * batched kernels below run on a one-member plan, so the results equal the batched path's
- * bitwise.  `scratch` must be 256-byte aligned and at least spd_fwd_scratch_bytes(desc) long;
+ * Three launches on `stream`: a one-block one that makes the previous call's cloud-top level set
+ * (shortwave_radiation.py:62-68: the cloud tops of every column) this call's prediction; then every
+ * column whole in one pass (all terms, verify_tendencies when on, every output); then a fixup that
+ * returns at once when the prediction held.  Under SPD_NO_SPECULATION a light launch over every
+ * column forms the level set first instead, and there is no fixup.  They are the batched kernels
+ * below run on a one-member plan, so the results equal the batched path's bitwise.  `scratch` must be 256-byte aligned and at least spd_fwd_scratch_bytes(desc) long;
  * it is initialised by the call. */
 int spd_fwd(const spd_desc_t* desc, const spd_vgrid_t* vgrid, const spd_params_t* params,
             const spd_inputs_t* in, const spd_outputs_t* out, void* scratch,
@@ -299,11 +299,11 @@ int spd_ensemble_plan(const spd_class_t* classes, int nclasses, const spd_member
                       int nmembers, void* plan_host, void* plan_device, size_t plan_bytes,
                       spd_plan_info_t* info);
 
-/* Runs every member.  grid_blocks = 0 picks SMs x resident blocks for both launches (each
- * block strides over the tile list: the fastest form on an otherwise idle GPU); a positive
- * value sets the second launch's persistent grid (the autotuner's knob); SPD_GRID_PER_TILE
- * launches one block per tile for both launches, which shares the GPU better with concurrent
- * kernels (a late-starting persistent block still owns its whole stride of tiles). */
+/* Runs every member.  grid_blocks = 0 picks the launch shape; a positive value sets the fused
+ * launch's persistent grid, whose blocks stride over the tile list (the autotuner's knob);
+ * SPD_GRID_PER_TILE launches one block per tile, which also shares the GPU better with concurrent
+ * kernels (a late-starting persistent block still owns its whole stride of tiles) and is what 0
+ * picks. */
 #define SPD_GRID_PER_TILE (-1)
 int spd_ensemble_fwd(const spd_class_t* classes, int nclasses, void* plan_device,
                      const spd_plan_info_t* info, int grid_blocks, void* stream);

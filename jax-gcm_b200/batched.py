@@ -1,5 +1,5 @@
 """Batched ragged ensembles: many grid instances of mixed resolution and level count run in
-one pair of persistent launches (``spd_ensemble_fwd``), optionally captured in a CUDA graph.
+one fused launch (``spd_ensemble_fwd``), optionally captured in a CUDA graph.
 
 Each member gives the same tendencies as ``SpeedyPhysics.compute_tendencies`` on it alone
 (jcm/physics/speedy/speedy_physics.py:88-127); the batching has no reference counterpart.
@@ -143,15 +143,15 @@ class Ensemble:
         return int(self.plan[off:off + 4].view(torch.int32).item())
 
     def autotune(self, candidates=None, reps=5):
-        """Picks the launch shape by timing the candidates (CUDA events): persistent grids of
-        0 (SMs x resident blocks), 1-4 blocks per SM, or one block per tile
-        (``_lib.GRID_PER_TILE``); cached per ensemble signature."""
+        """Picks the launch shape by timing the candidates (CUDA events): one block per tile
+        (0, the default) or persistent grids of 1-4 blocks per SM; cached per ensemble
+        signature."""
         sig = self.signature()
         if sig in _TUNE_CACHE:
             self.grid_blocks = _TUNE_CACHE[sig]
             return self.grid_blocks
         sms = torch.cuda.get_device_properties(self.device).multi_processor_count
-        cands = candidates or [0, sms, 2 * sms, 3 * sms, 4 * sms, _lib.GRID_PER_TILE]
+        cands = candidates or [0, sms, 2 * sms, 3 * sms, 4 * sms]
         best, best_ms = 0, float("inf")
         for gb in cands:
             self.forward(gb)

@@ -5,10 +5,10 @@
 // one cross-column dependency is the instance's cloud-top level set S (an OR over the columns'
 // clip(icltop, 0, kx-1), shortwave_radiation.py:62-68), which the shortwave of every column
 // reads.  By default the call predicts S from the previous call on the same scratch:
-//   1. ensemble_fused: every column whole, in one pass, its shortwave using the predicted S
-//      while the columns OR their own cloud tops into the true S; the last block to finish
-//      compares the two and keeps the true one as the next prediction;
-//   2. ensemble_fixup: returns at once when the prediction held, else computes every column
+//   1. ensemble_begin: the last call's true S becomes this call's prediction;
+//   2. ensemble_fused: every column whole, in one pass, its shortwave using the predicted S
+//      while the columns OR their own cloud tops into the true S;
+//   3. ensemble_fixup: returns at once when the prediction held, else computes every column
 //      again with the true S.
 // With SPD_NO_SPECULATION (or SPD_ACCUMULATE_DIAGNOSTICS) a light launch forms S first
 // (ensemble_levelset) and ensemble_fused reads it.  One thread owns one column
@@ -20,7 +20,7 @@
 
 namespace spd {
 
-constexpr size_t kHeaderBytes = 256;  // launch words and level-set state, padding
+constexpr size_t kHeaderBytes = 256;  // level-set state, padding
 
 static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
@@ -115,8 +115,7 @@ Consts make_consts(const spd_desc_t* d, const spd_vgrid_t* vg, const spd_params_
 // The forward of one instance: the batched kernels over an implicit one-member plan passed
 // by value (tile t = columns t*kNT ..), one block per tile.  The plain and the batched path
 // therefore run the same code and agree bitwise.  `header` is the instance's 256-byte scratch
-// header: words 0-1 the launch words, 4-6 the level-set state T, R, P (stride 1), 7 the
-// cumulative count of redone calls; words 0-5 are cleared by every call, P and the count kept.
+// header: words 4 and 6 the level-set state T and P, 7 the cumulative count of redone calls.
 int dispatch_fwd(const ConstsD& CD, int kx, const spd_inputs_t& in, const spd_outputs_t& out,
                  uint32_t* header, cudaStream_t st, cudaEvent_t marker) {
   if (kx != 7 && kx != 8 && kx != 16) return SPD_ERR_KX;
@@ -132,13 +131,11 @@ int dispatch_fwd(const ConstsD& CD, int kx, const spd_inputs_t& in, const spd_ou
   T.single.S = header + 4;
   T.single.ls_stride = 1;
   T.nmembers = 1;
-  T.launch = header;
   T.redone = header + 7;
   const bool speculate =
       (CD.K.flags & (SPD_ACCUMULATE_DIAGNOSTICS | SPD_NO_SPECULATION)) == 0;
   const int ntiles = (CD.K.C + kNT - 1) / kNT;
-  return launch_forward(A, T, ntiles, kx, SPD_GRID_PER_TILE, speculate, 6 * sizeof(uint32_t),
-                        st, marker);
+  return launch_forward(A, T, ntiles, kx, SPD_GRID_PER_TILE, speculate, st, marker);
 }
 
 int preload_ensemble();

@@ -4,15 +4,16 @@
 // A member is one grid instance (its own arrays, ix*il columns, kx levels).  The plan splits
 // every member into tiles of kNT consecutive columns (a tile never straddles members), ordered
 // by level count (16-level tiles first, the heavier work), and keeps per member the field
-// pointers and its cloud-top level-set words (P: the prediction, T: the true set, R: missed).
+// pointers and its cloud-top level-set words (P: the prediction, T: the true set).
 // The one cross-column dependency is the level set S (shortwave_radiation.py:62-68).  Two
 // launch forms:
-//   speculating (the default): the fused launch runs every column whole, in one pass, with
-//     each member's predicted set P (the previous call's) while the columns OR their own cloud
-//     tops into T; its last block compares T with P and marks the members that missed (R).
-//     The fixup launch, a programmatic dependent launch of one resident wave, computes the
-//     missed members again with their true set; when none missed its blocks read one word
-//     and return.
+//   speculating (the default): a one-block launch makes the level set that the last call's columns
+//     formed (T) each member's prediction (P) and clears T; the fused launch runs every column
+//     whole, in one pass, with P while the columns OR their own cloud tops into T; the fixup launch
+//     compares the two and computes the members that missed again with T.  The fused and the fixup
+//     launch are programmatic dependent launches: the fused one's blocks compute their first half
+//     while the first launch runs, and the fixup's, one resident wave, start as the fused one's
+//     retire and return after comparing the words when no member missed.
 //   level set first (accumulating calls, which must not add a column's diagnostics twice, and
 //     calls that ask for no prediction): a light launch forms every member's S from the
 //     cloud-top part of every column, then the fused launch reads it.
@@ -93,43 +94,19 @@ __device__ __forceinline__ uint32_t fused_column(const ConstsD& CD, float* sm,
   return fused_process<KX>(CD, sm, m.in, m.out, S, c, m.C, m.il);
 }
 
-// The end of a fused launch, in its last block to finish: every member's P becomes the level
-// set its columns formed (T); when speculating, R marks the members whose prediction P missed,
-// the launch word ANY says whether any did, and the cumulative count grows by their number.
-// `words` are two words of the block's shared memory that the columns no longer use (the
-// fused launch declares no static shared memory: one more word would leave room for three
-// blocks per SM instead of four at 16 levels).
-__device__ __forceinline__ void finish_fused(const TileSource& T, bool speculate,
-                                             uint32_t* words) {
-  uint32_t& last = words[0];
-  uint32_t& redo_block = words[1];
-  __syncthreads();  // every warp of this block has issued its level-set ORs and left the arena
-  if (threadIdx.x == 0) {
-    __threadfence();
-    last = atomicAdd(T.launch + LW_DONE, 1u) == gridDim.x - 1;
-    redo_block = 0;
-  }
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
+// Start of a call: the level set that the last call's columns formed (T) becomes each member's
+// prediction (P), and T starts at zero.  One block.  (Before, a memset cleared T and the fused
+// launch's last block, found by an atomic count that every block waited for, compared T with P:
+// T21 22.7 -> 17.5 us on the device, T425 with 8 levels 160 -> 151 us, with 16 levels 278 ->
+// 273 us.)
+__global__ void __launch_bounds__(kNT) ensemble_begin(const __grid_constant__ TileSource T) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int nm = T.members ? T.nmembers : 1;
-  uint32_t redo = 0;
   for (int i = threadIdx.x; i < nm; i += blockDim.x) {
-    const MemberDev& m = T.members ? T.members[i] : T.single;
-    volatile uint32_t* S = m.S;
-    const uint32_t t = S[LS_T * m.ls_stride];
-    if (speculate) {
-      const uint32_t r = t != S[LS_P * m.ls_stride] ? 1u : 0u;
-      S[LS_R * m.ls_stride] = r;
-      redo += r;
-    }
-    S[LS_P * m.ls_stride] = t;
-  }
-  if (redo) atomicAdd(&redo_block, redo);
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    T.launch[LW_ANY] = redo_block ? 1u : 0u;
-    if (redo_block) atomicAdd(T.redone, redo_block);
+    uint32_t* S = T.members ? T.members[i].S : T.single.S;
+    const int stride = T.members ? T.members[i].ls_stride : T.single.ls_stride;
+    S[LS_P * stride] = S[LS_T * stride];
+    S[LS_T * stride] = 0u;
   }
 }
 
@@ -158,30 +135,38 @@ __global__ void __launch_bounds__(kNT, 4) ensemble_fused(const __grid_constant__
   }
   // the fixup launch may start as this one's blocks retire; it waits for completion
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  finish_fused(T, speculate != 0, reinterpret_cast<uint32_t*>(sm));
 }
 
-// Fixup launch after a speculating fused launch: the members whose prediction missed (R set)
-// are computed again with their true level set (P, now equal to T).  In the common case no
-// member missed and every block returns after reading one word.
+// Fixup launch after a speculating fused launch: the members whose prediction P missed the level
+// set T that their columns formed are computed again with T.  In the common case none missed and
+// every block returns after comparing the words.
 __global__ void __launch_bounds__(kNT, 4) ensemble_fixup(const __grid_constant__ ClassArgs A,
                                                          const __grid_constant__ TileSource T,
                                                          int ntiles) {
   extern __shared__ float sm[];
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  if (*reinterpret_cast<volatile uint32_t*>(T.launch + LW_ANY) == 0u) return;
+  const int nm = T.members ? T.nmembers : 1;
+  int missed = 0;
+  for (int i = threadIdx.x; i < nm; i += kNT) {
+    const volatile uint32_t* S = T.members ? T.members[i].S : T.single.S;
+    const int stride = T.members ? T.members[i].ls_stride : T.single.ls_stride;
+    missed += S[LS_T * stride] != S[LS_P * stride];
+  }
+  if (!__syncthreads_or(missed)) return;
+  if (blockIdx.x == 0 && missed) atomicAdd(T.redone, (uint32_t)missed);
   for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
     int col0;
     const MemberDev m = tile_member(T, t, col0);
-    if (*reinterpret_cast<volatile uint32_t*>(m.S + LS_R * m.ls_stride) == 0u) continue;
+    const volatile uint32_t* S = m.S;
+    if (S[LS_T * m.ls_stride] == S[LS_P * m.ls_stride]) continue;
     const int c = col0 + threadIdx.x;
-    const uint32_t* S = m.S + LS_P * m.ls_stride;
     if (c < m.C) {
       const ConstsD& CD = A.cls[m.cls];
+      const uint32_t* St = m.S + LS_T * m.ls_stride;
       switch (m.kx) {
-        case 16: fused_column<16>(CD, sm, m, S, c); break;
-        case 8: fused_column<8>(CD, sm, m, S, c); break;
-        default: fused_column<7>(CD, sm, m, S, c); break;
+        case 16: fused_column<16>(CD, sm, m, St, c); break;
+        case 8: fused_column<8>(CD, sm, m, St, c); break;
+        default: fused_column<7>(CD, sm, m, St, c); break;
       }
     }
   }
@@ -229,18 +214,19 @@ int residency(Residency& R) {
 }
 }  // namespace
 
-// Launches kernel<<<grid, kNT, smem, st>>>(args...) as a programmatic dependent launch: its
+// Launches kernel<<<grid, threads, smem, st>>>(args...) as a programmatic dependent launch: its
 // blocks may start as the previous launch's blocks retire (they wait on the device,
 // griddepcontrol.wait, before reading what that launch writes).
 template <class... KArgs, class... Args>
-static int launch_dependent(void (*kernel)(KArgs...), int grid, size_t smem, cudaStream_t st,
+static int launch_dependent(void (*kernel)(KArgs...), int grid, int threads, size_t smem,
+                            cudaStream_t st,
                             Args... args) {
   cudaLaunchAttribute attr;
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(kNT);
+  cfg.blockDim = dim3(threads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cfg.attrs = &attr;
@@ -250,48 +236,47 @@ static int launch_dependent(void (*kernel)(KArgs...), int grid, size_t smem, cud
 }
 
 int launch_forward(const ClassArgs& A, const TileSource& T, int ntiles, int kx_layout,
-                   int grid_blocks, bool speculate, size_t clear_bytes, cudaStream_t st,
-                   cudaEvent_t marker) {
+                   int grid_blocks, bool speculate, cudaStream_t st, cudaEvent_t marker) {
   Residency R;
   const int rc = residency(R);
   if (rc != SPD_OK) return rc;
   const int res_lvl = R.sms * R.lvl, res_cols = R.sms * R.cols[kx_layout];
   int grid_lvl, grid_cols, pf_lvl;
-  if (grid_blocks == SPD_GRID_PER_TILE) {
+  if (grid_blocks <= 0) {
     // one block per tile; the blocks resident beside this one run the next wave, so the tile
     // a wave ahead is the one to prefetch
     grid_lvl = grid_cols = ntiles;
     pf_lvl = res_lvl;
   } else {
     grid_lvl = std::min(res_lvl, ntiles);
-    grid_cols = std::min(grid_blocks > 0 ? grid_blocks : res_cols, ntiles);
+    grid_cols = std::min(grid_blocks, ntiles);
     pf_lvl = grid_lvl;
   }
   const size_t arena = arena_bytes(kx_layout);
-  // the fixup is one resident wave striding over the tiles: its blocks read one word and return
-  // when no prediction missed, and a grid of one block per tile spends microseconds on
+  // the fixup is one resident wave striding over the tiles: its blocks compare the level sets and
+  // return when no prediction missed, and a grid of one block per tile spends microseconds on
   // scheduling thousands of such blocks
   const int grid_fix = std::min(grid_cols, res_cols);
-  // the launch words and every member's T and R start at zero; P is kept from the last call
-  if (cudaMemsetAsync(T.launch, 0, clear_bytes, st) != cudaSuccess) return SPD_ERR_CUDA;
   int r;
   if (speculate) {
-    ensemble_fused<<<grid_cols, kNT, arena, st>>>(A, T, ntiles, 1);
+    ensemble_begin<<<1, kNT, 0, st>>>(T);
+    r = launch_dependent(ensemble_fused, grid_cols, kNT, arena, st, A, T, ntiles, 1);
+    if (r != SPD_OK) return r;
     if (marker) {  // timing hook: the fused launch apart, then the fixup in plain stream order
       if (cudaEventRecord(marker, st) != cudaSuccess) return SPD_ERR_CUDA;
       ensemble_fixup<<<grid_fix, kNT, arena, st>>>(A, T, ntiles);
-      r = SPD_OK;
     } else {
-      r = launch_dependent(ensemble_fixup, grid_fix, arena, st, A, T, ntiles);
+      r = launch_dependent(ensemble_fixup, grid_fix, kNT, arena, st, A, T, ntiles);
     }
   } else {
+    ensemble_begin<<<1, kNT, 0, st>>>(T);
     ensemble_levelset<<<grid_lvl, kNT, 0, st>>>(A, T, ntiles, pf_lvl);
     if (marker) {  // timing hook: the two launches apart, in plain stream order
       if (cudaEventRecord(marker, st) != cudaSuccess) return SPD_ERR_CUDA;
       ensemble_fused<<<grid_cols, kNT, arena, st>>>(A, T, ntiles, 0);
       r = SPD_OK;
     } else {
-      r = launch_dependent(ensemble_fused, grid_cols, arena, st, A, T, ntiles, 0);
+      r = launch_dependent(ensemble_fused, grid_cols, kNT, arena, st, A, T, ntiles, 0);
     }
   }
   if (r != SPD_OK) return r;
@@ -303,6 +288,7 @@ int preload_ensemble() {
   bool ok = cudaFuncGetAttributes(&a, ensemble_levelset) == cudaSuccess;
   ok &= cudaFuncGetAttributes(&a, ensemble_fused) == cudaSuccess;
   ok &= cudaFuncGetAttributes(&a, ensemble_fixup) == cudaSuccess;
+  ok &= cudaFuncGetAttributes(&a, ensemble_begin) == cudaSuccess;
   return ok ? SPD_OK : SPD_ERR_CUDA;
 }
 
@@ -392,10 +378,9 @@ int spd_ensemble_fwd_marked(const spd_class_t* classes, int nclasses, void* plan
   T.tiles = reinterpret_cast<const Tile*>(
       base + 256 + align256((size_t)info->nmembers * sizeof(MemberDev)));
   T.nmembers = info->nmembers;
-  T.launch = reinterpret_cast<uint32_t*>(base + info->levelset_offset);
-  T.redone = T.launch + (16 + 12 * (size_t)nw) / sizeof(uint32_t);
-  return launch_forward(A, T, info->ntiles, kx_layout, grid_blocks, speculate,
-                        16 + 8 * (size_t)nw, st, static_cast<cudaEvent_t>(event));
+  T.redone = reinterpret_cast<uint32_t*>(base + info->levelset_offset + 16 + 12 * (size_t)nw);
+  return launch_forward(A, T, info->ntiles, kx_layout, grid_blocks, speculate, st,
+                        static_cast<cudaEvent_t>(event));
 }
 
 }  // extern "C"

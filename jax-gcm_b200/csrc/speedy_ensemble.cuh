@@ -12,12 +12,9 @@
 namespace spd {
 
 // Level-set state of a member in the forward: S points at its accumulator T of the true level
-// set; R (S[ls_stride]) is its redo flag and P (S[2 ls_stride]) the level set its last forward
-// used, which the next forward predicts.
-enum { LS_T = 0, LS_R = 1, LS_P = 2 };
-// Words of one forward launch (TileSource::launch): the count of blocks done, whether any member
-// must be redone, and (cumulative, in the region's last 16 bytes) the members redone so far.
-enum { LW_DONE = 0, LW_ANY = 1 };
+// set; P (S[2 ls_stride]) is the level set its call uses, the one its last call formed.
+// (S[ls_stride] is unused.)
+enum { LS_T = 0, LS_P = 2 };
 
 struct MemberDev {
   spd_inputs_t in;
@@ -43,7 +40,6 @@ struct TileSource {
   const Tile* tiles;
   MemberDev single;
   int nmembers;
-  uint32_t* launch;   // the launch words
   uint32_t* redone;   // cumulative count of members redone
 };
 
@@ -71,16 +67,15 @@ __device__ __forceinline__ void prefetch_tile_rows(int nrows, RowFn row) {
   }
 }
 
-// The forward (speedy_ensemble.cu) over the ntiles tiles, after clearing the launch words and
-// every member's T and R (clear_bytes from T.launch).  speculate: the fused launch uses each
+// The forward (speedy_ensemble.cu) over the ntiles tiles.  speculate: the fused launch uses each
 // member's predicted level set P and a fixup launch redoes the members whose prediction missed;
 // otherwise a level-set launch forms every T before the fused launch reads it.  grid_blocks:
-// 0 = persistent grids of SMs x resident blocks; > 0 = the fused launch's persistent grid;
-// SPD_GRID_PER_TILE = one block per tile.  kx_layout is the largest level count among the
+// > 0 = the fused launch's persistent grid; 0 or SPD_GRID_PER_TILE = one block per tile (the
+// 61-member ensemble takes 150 us so, 161 us as a persistent grid of SMs x resident blocks,
+// whose blocks own unequal strides of 8- and 16-level tiles).  kx_layout is the largest level count among the
 // tiles (it sizes the fused launch's shared-memory arena).
 int launch_forward(const ClassArgs& A, const TileSource& T, int ntiles, int kx_layout,
-                   int grid_blocks, bool speculate, size_t clear_bytes, cudaStream_t st,
-                   cudaEvent_t marker);
+                   int grid_blocks, bool speculate, cudaStream_t st, cudaEvent_t marker);
 
 constexpr size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
@@ -109,7 +104,7 @@ __device__ __forceinline__ void prepass_tiles(const ClassArgs& A, const M* __res
 }
 
 // Device plan layout: header, member records, tile list, level-set region, solar tables.  The
-// level-set region: 16 bytes of launch words, then nw words each of every member's T, R and P
+// level-set region: 16 unused bytes, then nw words each of every member's T, an unused word and P
 // (nw = member count rounded up to 4), then 16 bytes whose first word counts the members the
 // forward redid (its prediction missed).
 struct PlanLayout {

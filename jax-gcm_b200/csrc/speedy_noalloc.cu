@@ -4,8 +4,7 @@
 // ctypes stub) that only forwards the state, forcing and tendency buffers handed to it, or a
 // process whose device memory is owned entirely by another runtime's pooling allocator.  This
 // entry point needs no scratch argument and performs no allocation: its scratch lives in the
-// fixed file-scope device array below.  The call's launch words and the instance's level-set
-// state take its first 256 bytes; the rest holds up to SPD_NOALLOC_MAX_IL rows of a
+// fixed file-scope device array below.  The instance's level-set state takes its first 256 bytes; the rest holds up to SPD_NOALLOC_MAX_IL rows of a
 // per-latitude table (the size limit of the entry point; the present kernels form each
 // column's solar row themselves and leave it unused).  Every GPU that loads the library keeps
 // that array (65,792 bytes) until the process exits.
@@ -25,7 +24,7 @@ int dispatch_fwd(const ConstsD& CD, int kx, const spd_inputs_t& in, const spd_ou
 
 namespace {
 
-constexpr size_t kNoallocHeader = 256;  // launch words, level-set state, padding
+constexpr size_t kNoallocHeader = 256;  // level-set state, padding
 constexpr size_t kNoallocBytes = kNoallocHeader + (size_t)SPD_NOALLOC_MAX_IL * sizeof(spd::ZonalRow);
 
 // The shared scratch.  In host code this name is only a host-side stand-in for the symbol;
@@ -70,8 +69,8 @@ extern "C" int spd_fwd_noalloc(const spd_desc_t* desc, const spd_vgrid_t* vgrid,
   spd::ConstsD CD;
   CD.K = spd::make_consts(desc, vgrid, params);
   CD.D = spd::derive_constants(desc, vgrid, params);
-  // The array keeps the previous call's contents: the call clears the words that must start
-  // at zero itself, and keeps the previous call's level set as its prediction (a prediction
+  // The array keeps the previous call's contents: the call clears the word that must start
+  // at zero itself, and takes the previous call's level set as its prediction (a prediction
   // that misses, e.g. after another instance's call, costs a second pass, never a wrong
   // result).
   return spd::dispatch_fwd(CD, desc->kx, *in, *out, static_cast<uint32_t*>(scratch), st,
