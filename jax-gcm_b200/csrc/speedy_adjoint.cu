@@ -3,15 +3,15 @@
 //
 // Launch 1 is the forward's cloud-top pre-pass over the tile list of speedy_ensemble.cuh (each
 // member's level set S and per-latitude solar table: neither carries a derivative).  Launch 2
-// runs one thread per column, one warp per block: the reverse pass of speedy_vjp_smem.cuh
+// runs one thread per column, one block per tile: the reverse pass of speedy_vjp_smem.cuh
 // recomputes the column's forward and walks its terms backwards, writing the state gradients;
 // the 12 parameter gradients are summed per thread, then per warp, then added to the tile's
 // member with one coalesced atomic.  A single instance is a one-member plan written into its
 // scratch by a small kernel, so it runs exactly the ensemble's instructions.
 //
 // Measured (the whole call, against the fully unrolled reverse pass with its arrays in registers
-// and local memory that this replaces): T425 with 16 levels 3,191 -> 1,034 us, T170 with 16
-// levels and verify 578 -> 206 us, T85 with 16 levels 129 -> 57 us.
+// and local memory that this replaces): T425 with 16 levels 3,191 -> 942 us, T170 with 16
+// levels and verify 578 -> 213 us, T85 with 16 levels 129 -> 57 us.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -68,30 +68,34 @@ __global__ void __launch_bounds__(kBlock)
   prepass_tiles(A, members, tiles, ntiles);
 }
 
-// The adjoint launch: one thread per column (speedy_vjp_smem.cuh), one warp per block with its
-// level arrays in `sm`, so that no warp waits for another and a finished one makes room at once.
-// At 16 levels an arena is 18,432 bytes, which with the 1,024 reserved per block is exactly a
-// twelfth of an SM's shared memory: twelve warps, which 168 registers allow as well.  The threads
-// past a member's last column run that column again and store nothing, so that every warp is whole
-// (the convection's reverse votes).
-// Two register budgets: 168 (three warps per scheduler), or 255 (two), which spills nothing and is
-// the faster where two warps per scheduler hold the whole batch (T85 with 16 levels, 1,024 warps:
-// 60 against 66 us; T170, 4,096 warps: 209 against 194 us).  Both give the same bits, so a
-// member's gradients do not depend on the batch that carried it.
+// The adjoint launch: one thread per column (speedy_vjp_smem.cuh), one block per tile with its
+// level arrays in `sm`, no barrier.  The threads past a member's last column run that column again
+// and store nothing, so that every warp is whole (the convection's reverse votes).  Blocks of one
+// warp, which make room as soon as their columns are done, are no faster: a block's four warps
+// start together and share what they fetch of the code (T425 with 16 levels, 32 / 64 / 128 / 384
+// threads: 1,029 / 972 / 942 / 1,001 us; with 8 levels 563 / 537 / 500 / 515 us).  Barriers at the
+// stage boundaries cost 0.5 %.
+// Three register budgets, which give the same bits, so that a member's gradients do not depend on
+// the batch that carried it:
+//  - 168 (twelve warps per SM), what the arena of 16 levels leaves room for (73,728 bytes and the
+//    1,024 reserved per block, three blocks);
+//  - 128 (sixteen) where the batch has at most 8 levels, whose arenas do not bind (T425 with 8
+//    levels 458 against 500 us; the spills of 128 registers cost 16 levels 993 against 942 us, and
+//    96 registers with twenty warps 442 us at T425 but 110 against 96 us at T170);
+//  - 255 (eight), which spills next to nothing, where two warps per scheduler hold the whole batch
+//    (T85 with 16 levels, 1,024 warps: 60 against 66 us; T170, 4,096 warps: 209 against 194 us).
 template <int kWarpsPerSm>
-__global__ void __launch_bounds__(kVjpThreads, kWarpsPerSm)
+__global__ void __launch_bounds__(kNT, kWarpsPerSm / (kNT / 32))
     ensemble_adjoint(const __grid_constant__ ClassArgs A,
                      const VjpMemberDev* __restrict__ members, const Tile* __restrict__ tiles,
                      int ntiles) {
-  constexpr int kPerTile = kNT / kVjpThreads;
   extern __shared__ float sm[];
-  for (int b = blockIdx.x; b < ntiles * kPerTile; b += gridDim.x) {
-    const Tile tl = tiles[b / kPerTile];
+  for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
+    const Tile tl = tiles[t];
     const VjpMemberDev* m = members + tl.member;
-    const int C = m->C, col0 = tl.col0 + (b % kPerTile) * kVjpThreads;
-    if (col0 >= C) continue;
-    const bool valid = col0 + (int)threadIdx.x < C;
-    const int c = valid ? col0 + (int)threadIdx.x : C - 1;
+    const int C = m->C, at = tl.col0 + (int)threadIdx.x;
+    const bool valid = at < C;
+    const int c = valid ? at : C - 1;
     float pacc[SPD_NUM_DIFF_PARAMS];
 #pragma unroll
     for (int j = 0; j < SPD_NUM_DIFF_PARAMS; ++j) pacc[j] = 0.0f;
@@ -121,11 +125,11 @@ static int allow_arena(int* sms = nullptr) {
   if (!count[dev]) {
     const int bytes = (int)vjp_arena_bytes(SPD_MAX_KX);
     int n = 0;
-    if (cudaFuncSetAttribute(ensemble_adjoint<12>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             bytes) != cudaSuccess ||
-        cudaFuncSetAttribute(ensemble_adjoint<8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             bytes) != cudaSuccess ||
-        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    for (auto* kernel : {ensemble_adjoint<8>, ensemble_adjoint<12>, ensemble_adjoint<16>})
+      if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) !=
+          cudaSuccess)
+        return SPD_ERR_CUDA;
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
       return SPD_ERR_CUDA;
     count[dev] = n;
   }
@@ -156,8 +160,8 @@ int preload_adjoint() {
   bool ok = true;
   ok &= cudaFuncGetAttributes(&a, vjp_single_plan) == cudaSuccess;
   ok &= cudaFuncGetAttributes(&a, ensemble_vjp_prepass) == cudaSuccess;
-  ok &= cudaFuncGetAttributes(&a, ensemble_adjoint<12>) == cudaSuccess;
-  ok &= cudaFuncGetAttributes(&a, ensemble_adjoint<8>) == cudaSuccess;
+  for (auto* kernel : {ensemble_adjoint<8>, ensemble_adjoint<12>, ensemble_adjoint<16>})
+    ok &= cudaFuncGetAttributes(&a, kernel) == cudaSuccess;
   return ok && allow_arena() == SPD_OK ? SPD_OK : SPD_ERR_CUDA;
 }
 
@@ -171,8 +175,7 @@ static int launch_ensemble_vjp(const ClassArgs& A, int kx_layout, char* base, in
   // Default: one block per tile.  The blocks are short (one tile's columns each), so the SMs
   // turn over often and a higher-priority stream's kernels (a forward batch) get them within
   // one block's time; a persistent grid would hold every SM until the whole batch is done.
-  const int grid =
-      (grid_blocks > 0 ? std::min(grid_blocks, ntiles) : ntiles) * (kNT / kVjpThreads);
+  const int grid = grid_blocks > 0 ? std::min(grid_blocks, ntiles) : ntiles;
   const int grid_pre = std::min(ntiles, 65535);
   int sms = 0;
   if (allow_arena(&sms) != SPD_OK) return SPD_ERR_CUDA;
@@ -180,10 +183,10 @@ static int launch_ensemble_vjp(const ClassArgs& A, int kx_layout, char* base, in
     return SPD_ERR_CUDA;
   ensemble_vjp_prepass<<<grid_pre, kBlock, 0, st>>>(A, md, tl, ntiles);
   const size_t arena = vjp_arena_bytes(kx_layout);
-  if (grid <= 8 * sms)
-    ensemble_adjoint<8><<<grid, kVjpThreads, arena, st>>>(A, md, tl, ntiles);
-  else
-    ensemble_adjoint<12><<<grid, kVjpThreads, arena, st>>>(A, md, tl, ntiles);
+  auto* kernel = grid * (kNT / 32) <= 8 * sms ? ensemble_adjoint<8>
+                 : kx_layout > 8              ? ensemble_adjoint<12>
+                                              : ensemble_adjoint<16>;
+  kernel<<<grid, kNT, arena, st>>>(A, md, tl, ntiles);
   return cudaGetLastError() == cudaSuccess ? SPD_OK : SPD_ERR_CUDA;
 }
 

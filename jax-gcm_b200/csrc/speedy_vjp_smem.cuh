@@ -36,17 +36,9 @@ namespace spd {
 
 enum { V_T, V_Q, V_QS, V_TB, V_QB, V_S0, V_S1, V_S2, V_S3, kVjpArrays };
 
-constexpr int kVjpThreads = 32;  // threads per block = columns per block
-
 constexpr size_t vjp_arena_bytes(int kx) {
-  return (size_t)kVjpArrays * kx * kVjpThreads * sizeof(float);
+  return (size_t)kVjpArrays * kx * kNT * sizeof(float);
 }
-
-// Per-thread level array: element k of this thread lives at p[k * kVjpThreads].
-struct VLv {
-  float* p;
-  __device__ __forceinline__ float& operator[](int k) const { return p[k * kVjpThreads]; }
-};
 
 // Packed pairs without the subnormal flush of speedy_pk.cuh, and with a fused multiply-add.  No
 // sum below has a product for an operand where a fused multiply-add could take its place (ptxas
@@ -365,9 +357,9 @@ __device__ __forceinline__ void column_vjp_smem(const ConstsD& CD, float* sm,
   const spd_vgrid_t& vg = K.vg;
   constexpr int B = KX - 1;
   const size_t C = (size_t)Ci;
-  auto arr = [&](int a) { return VLv{sm + (size_t)a * KX * kVjpThreads + threadIdx.x}; };
-  const VLv T = arr(V_T), Q = arr(V_Q), QS = arr(V_QS), TB = arr(V_TB), QB = arr(V_QB);
-  const VLv S0 = arr(V_S0), S1 = arr(V_S1), S2 = arr(V_S2), S3 = arr(V_S3);
+  auto arr = [&](int a) { return Lv{sm + (size_t)a * KX * kNT + threadIdx.x}; };
+  const Lv T = arr(V_T), Q = arr(V_Q), QS = arr(V_QS), TB = arr(V_TB), QB = arr(V_QB);
+  const Lv S0 = arr(V_S0), S1 = arr(V_S1), S2 = arr(V_S2), S3 = arr(V_S3);
   const bool verify = (K.flags & SPD_FUSE_VERIFY) != 0;
   const VjpColumn col{field(&m->in.geopotential) + c, field(&m->ct.temperature) + c,
                       field(&m->ct.specific_humidity) + c, C};
@@ -376,10 +368,11 @@ __device__ __forceinline__ void column_vjp_smem(const ConstsD& CD, float* sm,
   // two cotangents' levels, then the surface fields.
   {
     const int lane = threadIdx.x & 31, level = lane & 15;
-    const float* row = (lane < 16 ? col.ct_t : col.ct_q) - lane;
+    const int c0 = __shfl_sync(0xffffffffu, c, 0);  // the warp's first column
+    const float* row = (lane < 16 ? col.ct_t : col.ct_q) - c + c0;
     if (level < KX) asm volatile("prefetch.global.L2 [%0];" ::"l"(row + level * C));
     const float* const* fields = &m->in.alb0;  // alb0 .. phis0
-    if (lane < 9) asm volatile("prefetch.global.L2 [%0];" ::"l"(field(fields + lane) + (c - lane)));
+    if (lane < 9) asm volatile("prefetch.global.L2 [%0];" ::"l"(field(fields + lane) + c0));
   }
 
   // ---- forward: humidity, convection, condensation, clouds ----------------------------------
@@ -846,7 +839,7 @@ __device__ __forceinline__ void column_vjp_smem(const ConstsD& CD, float* sm,
   // ---- clouds' reverse (scalars), vertical diffusion's reverse, both level by level -----------
   // From here S0 is the phi adjoint, S1 the qsat adjoint; S2 holds the relative humidity and S3
   // the running maximum of the cloud cover's candidates.
-  const VLv PB = S0, XB = S1, RHs = S2, PM = S3;
+  const Lv PB = S0, XB = S1, RHs = S2, PM = S3;
   auto dq_b = [&](int k) {
     return ((limited >> k) & 1u) ? 0.0f : col.at(col.ct_q, k) * K.q_tend_scale;
   };
@@ -1097,7 +1090,7 @@ __device__ __forceinline__ void column_vjp_smem(const ConstsD& CD, float* sm,
       const float fmass = D.fm0 * fpsa * mn;
       const float cbmf = convects ? fmass : 0.0f * fmass;
       const float fus = fmass * seB, fuq = fmass * qmax, fds = fmass * sb, fdq = fmass * qb;
-      const VLv FM = S2;
+      const Lv FM = S2;
       auto e_of = [&](float cqk, int k) {
         return (((limited >> k) & 1u) ? 0.0f : cqk * K.q_tend_scale) * vg.grdsig[k] * rpsa;
       };

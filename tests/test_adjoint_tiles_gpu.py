@@ -1,6 +1,6 @@
 """The adjoint's tiles at the sizes where they can go wrong: one column, less than a warp, one
 column past a tile, a last tile of a few columns; gradients written over the cotangents; and the
-two register budgets, chosen by the batch's warps, bit for bit.
+register budgets, chosen by the batch's warps and levels, bit for bit.
 
 Each column against the host builds of the hand-written reverse pass, with the bar of
 tests/test_adjoint_gpu.py: 1e-4 of the field's largest gradient, or three times the host float32
@@ -107,11 +107,12 @@ def test_gradients_may_overwrite_the_cotangents(pkg):
     assert torch.equal(psa, want.normalized_surface_pressure)
 
 
-def test_register_budgets_give_the_same_bits(pkg):
-    """16,384 columns run two warps per scheduler, the 65,536 columns that contain them three: the
-    same columns' state gradients are equal in every bit."""
+@pytest.mark.parametrize("kx", [7, 8, 16])
+def test_register_budgets_give_the_same_bits(pkg, kx):
+    """16,384 columns run two warps per scheduler, the 65,536 columns that contain them three or
+    four: the same columns' state gradients are equal in every bit."""
     import torch
-    kx, il = 16, 256
+    il = 256
     inst = pkg.synthetic.land_instance(77, 256, il, kx)
     state, forcing, geom, date = pkg.instance_to_device(inst, "cuda")
     phys = pkg.SpeedyPhysics(diagnostics=False, fuse_verify=True, time_step=1800.0)
