@@ -1,13 +1,13 @@
 // speedy_adjoint.cu -- the adjoint of the forward: one instance (spd_vjp) or a ragged ensemble
-// of them (spd_ensemble_vjp), both through the same two kernels.
+// of them (spd_ensemble_vjp), both through the same three launches (the first clears what they add to).
 //
-// Launch 1 is the forward's cloud-top pre-pass over the tile list of speedy_ensemble.cuh (each
-// member's level set S and per-latitude solar table: neither carries a derivative).  Launch 2
+// Launch 2 is the forward's cloud-top pre-pass over the tile list of speedy_ensemble.cuh (each
+// member's level set S and per-latitude solar table: neither carries a derivative).  Launch 3
 // runs one thread per column, one block per tile: the reverse pass of speedy_vjp_smem.cuh
 // recomputes the column's forward and walks its terms backwards, writing the state gradients;
 // the 12 parameter gradients are summed per thread, then per warp, then added to the tile's
-// member with one coalesced atomic.  A single instance is a one-member plan written into its
-// scratch by a small kernel, so it runs exactly the ensemble's instructions.
+// member with one coalesced atomic.  A single instance is one member given by value to the same
+// kernels.
 //
 // Measured (the whole call, against the fully unrolled reverse pass with its arrays in registers
 // and local memory that this replaces): T425 with 16 levels 3,191 -> 942 us, T170 with 16
@@ -54,22 +54,50 @@ __device__ __forceinline__ void warp_add_params(const float* pacc, float* params
   if ((lane & 1) == 0 && j < SPD_NUM_DIFF_PARAMS) atomicAdd(params + j, v[0]);
 }
 
-// ---- ensemble ----
+// Start of a call: every member's level set and parameter gradients at zero.  One block.
+__global__ void __launch_bounds__(kBlock) vjp_begin(const __grid_constant__ VjpSource T) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const int nm = T.members ? T.nmembers : 1;
+  for (int i = threadIdx.x; i < nm * (SPD_NUM_DIFF_PARAMS + 1); i += blockDim.x) {
+    const int j = i % (SPD_NUM_DIFF_PARAMS + 1);
+    const VjpMemberDev* m = T.members ? T.members + i / (SPD_NUM_DIFF_PARAMS + 1) : nullptr;
+    if (j == SPD_NUM_DIFF_PARAMS)
+      *(m ? m->S : T.single.S) = 0u;
+    else
+      (m ? m->gr.params : T.single.gr.params)[j] = 0.0f;
+  }
+}
+
+// Pre-pass: each member's level set and solar table.  It may start beside vjp_begin, and waits
+// for it before it adds to a level set.
+template <int KX>
+__device__ __forceinline__ uint32_t prepass_bit(const Consts& K, const spd_inputs_t& in, int c,
+                                                int C, uint32_t* S, ZonalRow* table, int il) {
+  if (c < il) table[c] = zonal_row(K.tyear, __ldg(in.sia + c), __ldg(in.coa + c));
+  return c < C ? prepass_column<KX>(K, in, c, C) : 0u;
+}
 __global__ void __launch_bounds__(kBlock)
     ensemble_vjp_prepass(const __grid_constant__ ClassArgs A,
-                         const VjpMemberDev* __restrict__ members,
-                         const Tile* __restrict__ tiles, int ntiles) {
-  // the adjoint launch accumulates each member's parameter gradients: zero them here
+                         const __grid_constant__ VjpSource T, int ntiles) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-    const Tile tl = tiles[t];
-    if (tl.col0 == 0 && threadIdx.x < SPD_NUM_DIFF_PARAMS)
-      members[tl.member].gr.params[threadIdx.x] = 0.0f;
+    const Tile tl = T.members ? T.tiles[t] : Tile{0, t * kNT};
+    const VjpMemberDev& m = T.members ? T.members[tl.member] : T.single;
+    const Consts& K = A.cls[m.cls].K;
+    const int c = tl.col0 + threadIdx.x;
+    uint32_t bit;
+    switch (m.kx) {  // uniform per block
+      case 16: bit = prepass_bit<16>(K, m.in, c, m.C, m.S, m.table, m.il); break;
+      case 8: bit = prepass_bit<8>(K, m.in, c, m.C, m.S, m.table, m.il); break;
+      default: bit = prepass_bit<7>(K, m.in, c, m.C, m.S, m.table, m.il); break;
+    }
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    or_level_set_warp(bit, m.S);
   }
-  prepass_tiles(A, members, tiles, ntiles);
 }
 
 // The adjoint launch: one thread per column (speedy_vjp_smem.cuh), one block per tile with its
-// level arrays in `sm`, no barrier.  The threads past a member's last column run that column again
+// level arrays in `sm` and no barrier but around its member's record.  The threads past a member's last column run that column again
 // and store nothing, so that every warp is whole (the convection's reverse votes).  Blocks of one
 // warp, which make room as soon as their columns are done, are no faster: a block's four warps
 // start together and share what they fetch of the code (T425 with 16 levels, 32 / 64 / 128 / 384
@@ -86,30 +114,36 @@ __global__ void __launch_bounds__(kBlock)
 //    (T85 with 16 levels, 1,024 warps: 60 against 66 us; T170, 4,096 warps: 209 against 194 us).
 template <int kWarpsPerSm>
 __global__ void __launch_bounds__(kNT, kWarpsPerSm / (kNT / 32))
-    ensemble_adjoint(const __grid_constant__ ClassArgs A,
-                     const VjpMemberDev* __restrict__ members, const Tile* __restrict__ tiles,
+    ensemble_adjoint(const __grid_constant__ ClassArgs A, const __grid_constant__ VjpSource T,
                      int ntiles) {
   extern __shared__ float sm[];
+  __shared__ VjpMemberDev m;
+  constexpr int kWords = sizeof(VjpMemberDev) / sizeof(uint64_t);
+  static_assert(kWords <= kNT && sizeof(VjpMemberDev) % sizeof(uint64_t) == 0, "one copy per thread");
   for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-    const Tile tl = tiles[t];
-    const VjpMemberDev* m = members + tl.member;
-    const int C = m->C, at = tl.col0 + (int)threadIdx.x;
+    const Tile tl = T.members ? T.tiles[t] : Tile{0, t * kNT};
+    __syncthreads();  // the last tile's columns are done with its record
+    if (threadIdx.x < kWords) {
+      const uint64_t* from =
+          reinterpret_cast<const uint64_t*>(T.members ? T.members + tl.member : &T.single);
+      reinterpret_cast<uint64_t*>(&m)[threadIdx.x] = from[threadIdx.x];
+    }
+    __syncthreads();
+    const int C = m.C, at = tl.col0 + (int)threadIdx.x;
     const bool valid = at < C;
     const int c = valid ? at : C - 1;
     float pacc[SPD_NUM_DIFF_PARAMS];
 #pragma unroll
     for (int j = 0; j < SPD_NUM_DIFF_PARAMS; ++j) pacc[j] = 0.0f;
-    const ConstsD& CD = A.cls[m->cls];
-    const uint32_t S = *m->S;
-    const ZonalRow z = m->table[c % m->il];
-    switch (m->kx) {  // uniform per block
-      case 16: column_vjp_smem<16>(CD, sm, m, z, S, c, C, valid, pacc); break;
-      case 8: column_vjp_smem<8>(CD, sm, m, z, S, c, C, valid, pacc); break;
-      default: column_vjp_smem<7>(CD, sm, m, z, S, c, C, valid, pacc); break;
+    const ConstsD& CD = A.cls[m.cls];
+    switch (m.kx) {  // uniform per block
+      case 16: column_vjp_smem<16>(CD, sm, m, c, C, valid, pacc); break;
+      case 8: column_vjp_smem<8>(CD, sm, m, c, C, valid, pacc); break;
+      default: column_vjp_smem<7>(CD, sm, m, c, C, valid, pacc); break;
     }
 #pragma unroll
     for (int j = 0; j < SPD_NUM_DIFF_PARAMS; ++j) pacc[j] = valid ? pacc[j] : 0.0f;
-    warp_add_params(pacc, field(&m->gr.params));
+    warp_add_params(pacc, load_field(m.gr.params));
   }
 }
 
@@ -137,15 +171,6 @@ static int allow_arena(int* sms = nullptr) {
   return SPD_OK;
 }
 
-// The one-member plan of a single instance: its record and its tile list.
-__global__ void __launch_bounds__(kBlock) vjp_single_plan(const VjpMemberDev rec,
-                                                          VjpMemberDev* dst, Tile* tiles,
-                                                          int ntiles) {
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t == 0) *dst = rec;
-  for (; t < ntiles; t += gridDim.x * blockDim.x) tiles[t] = Tile{0, t * kNT};
-}
-
 struct OneMember {
   int ix, il;
 };
@@ -158,20 +183,16 @@ inline PlanLayout single_layout(const spd_desc_t* d) {
 int preload_adjoint() {
   cudaFuncAttributes a;
   bool ok = true;
-  ok &= cudaFuncGetAttributes(&a, vjp_single_plan) == cudaSuccess;
+  ok &= cudaFuncGetAttributes(&a, vjp_begin) == cudaSuccess;
   ok &= cudaFuncGetAttributes(&a, ensemble_vjp_prepass) == cudaSuccess;
   for (auto* kernel : {ensemble_adjoint<8>, ensemble_adjoint<12>, ensemble_adjoint<16>})
     ok &= cudaFuncGetAttributes(&a, kernel) == cudaSuccess;
   return ok && allow_arena() == SPD_OK ? SPD_OK : SPD_ERR_CUDA;
 }
 
-// Both launches over a plan already on the device (tiles at base + tiles_off).
-static int launch_ensemble_vjp(const ClassArgs& A, int kx_layout, char* base, int nmembers,
-                               int ntiles, size_t levelset_offset,
-                               size_t levelset_bytes, int grid_blocks, cudaStream_t st) {
-  const VjpMemberDev* md = reinterpret_cast<const VjpMemberDev*>(base + 256);
-  const size_t tiles_off = 256 + align256((size_t)nmembers * sizeof(VjpMemberDev));
-  const Tile* tl = reinterpret_cast<const Tile*>(base + tiles_off);
+// The three launches; each but the first may start while the one before it runs.
+static int launch_ensemble_vjp(const ClassArgs& A, int kx_layout, const VjpSource& T, int ntiles,
+                               int grid_blocks, cudaStream_t st) {
   // Default: one block per tile.  The blocks are short (one tile's columns each), so the SMs
   // turn over often and a higher-priority stream's kernels (a forward batch) get them within
   // one block's time; a persistent grid would hold every SM until the whole batch is done.
@@ -179,14 +200,14 @@ static int launch_ensemble_vjp(const ClassArgs& A, int kx_layout, char* base, in
   const int grid_pre = std::min(ntiles, 65535);
   int sms = 0;
   if (allow_arena(&sms) != SPD_OK) return SPD_ERR_CUDA;
-  if (cudaMemsetAsync(base + levelset_offset, 0, levelset_bytes, st) != cudaSuccess)
-    return SPD_ERR_CUDA;
-  ensemble_vjp_prepass<<<grid_pre, kBlock, 0, st>>>(A, md, tl, ntiles);
-  const size_t arena = vjp_arena_bytes(kx_layout);
+  vjp_begin<<<1, kBlock, 0, st>>>(T);
+  int rc = launch_dependent(ensemble_vjp_prepass, grid_pre, kBlock, 0, st, A, T, ntiles);
+  if (rc != SPD_OK) return rc;
   auto* kernel = grid * (kNT / 32) <= 8 * sms ? ensemble_adjoint<8>
                  : kx_layout > 8              ? ensemble_adjoint<12>
                                               : ensemble_adjoint<16>;
-  kernel<<<grid, kNT, arena, st>>>(A, md, tl, ntiles);
+  rc = launch_dependent(kernel, grid, kNT, vjp_arena_bytes(kx_layout), st, A, T, ntiles);
+  if (rc != SPD_OK) return rc;
   return cudaGetLastError() == cudaSuccess ? SPD_OK : SPD_ERR_CUDA;
 }
 
@@ -233,22 +254,18 @@ int spd_vjp(const spd_desc_t* desc, const spd_vgrid_t* vgrid, const spd_params_t
   ClassArgs A;
   A.cls[0].K = make_consts(desc, vgrid, params);
   A.cls[0].D = derive_constants(desc, vgrid, params);
-  VjpMemberDev rec;
-  rec.in = *in;
-  rec.ct = *ct;
-  rec.gr = *grads;
-  rec.C = desc->ix * desc->il;
-  rec.il = desc->il;
-  rec.kx = desc->kx;
-  rec.cls = 0;
-  rec.S = reinterpret_cast<uint32_t*>(base + L.levelset);
-  rec.table = reinterpret_cast<ZonalRow*>(base + L.tables);
-  VjpMemberDev* dst = reinterpret_cast<VjpMemberDev*>(base + L.members);
-  Tile* tiles = reinterpret_cast<Tile*>(base + L.tiles);
-  const int grid_init = std::min((L.ntiles + kBlock - 1) / kBlock, 1024);
-  vjp_single_plan<<<grid_init, kBlock, 0, st>>>(rec, dst, tiles, L.ntiles);
-  return launch_ensemble_vjp(A, desc->kx, base, 1, L.ntiles, L.levelset,
-                             align256(sizeof(uint32_t)), 0, st);
+  VjpSource T{};
+  T.single.in = *in;
+  T.single.ct = *ct;
+  T.single.gr = *grads;
+  T.single.C = desc->ix * desc->il;
+  T.single.il = desc->il;
+  T.single.kx = desc->kx;
+  T.single.cls = 0;
+  T.single.S = reinterpret_cast<uint32_t*>(base + L.levelset);
+  T.single.table = reinterpret_cast<ZonalRow*>(base + L.tables);
+  T.nmembers = 1;
+  return launch_ensemble_vjp(A, desc->kx, T, L.ntiles, 0, st);
 }
 
 size_t spd_ensemble_vjp_plan_bytes(const spd_vjp_member_t* members, int nmembers) {
@@ -309,12 +326,14 @@ int spd_ensemble_vjp(const spd_class_t* classes, int nclasses, void* plan_device
     A.cls[i].D = derive_constants(&classes[i].desc, &classes[i].vgrid, &classes[i].params);
     kx_layout = std::max(kx_layout, classes[i].desc.kx);
   }
-  // Default: one block per tile.  The blocks are short (one tile's columns each), so the SMs
-  // turn over often and a higher-priority stream's kernels (a forward batch) get them within
-  // one block's time; a persistent grid would hold every SM until the whole batch is done.
-  return launch_ensemble_vjp(A, kx_layout, static_cast<char*>(plan_device), info->nmembers,
-                             info->ntiles, info->levelset_offset, info->levelset_bytes,
-                             grid_blocks, static_cast<cudaStream_t>(stream));
+  char* base = static_cast<char*>(plan_device);
+  VjpSource T{};
+  T.members = reinterpret_cast<const VjpMemberDev*>(base + 256);
+  T.tiles = reinterpret_cast<const Tile*>(
+      base + 256 + align256((size_t)info->nmembers * sizeof(VjpMemberDev)));
+  T.nmembers = info->nmembers;
+  return launch_ensemble_vjp(A, kx_layout, T, info->ntiles, grid_blocks,
+                             static_cast<cudaStream_t>(stream));
 }
 
 }  // extern "C"

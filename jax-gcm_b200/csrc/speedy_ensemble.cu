@@ -214,27 +214,6 @@ int residency(Residency& R) {
 }
 }  // namespace
 
-// Launches kernel<<<grid, threads, smem, st>>>(args...) as a programmatic dependent launch: its
-// blocks may start as the previous launch's blocks retire (they wait on the device,
-// griddepcontrol.wait, before reading what that launch writes).
-template <class... KArgs, class... Args>
-static int launch_dependent(void (*kernel)(KArgs...), int grid, int threads, size_t smem,
-                            cudaStream_t st,
-                            Args... args) {
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(threads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
-  if (cudaLaunchKernelEx(&cfg, kernel, args...) != cudaSuccess) return SPD_ERR_CUDA;
-  return SPD_OK;
-}
-
 int launch_forward(const ClassArgs& A, const TileSource& T, int ntiles, int kx_layout,
                    int grid_blocks, bool speculate, cudaStream_t st, cudaEvent_t marker) {
   Residency R;

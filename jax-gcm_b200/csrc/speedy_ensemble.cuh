@@ -1,7 +1,6 @@
 // speedy_ensemble.cuh -- what the batched forward and the batched adjoint share: the tile
-// list over ragged members, the per-class constants passed by value, and the adjoint's
-// cloud-top pre-pass over all tiles (each member's level set and per-latitude solar table;
-// the forward forms both in its first launch).
+// list over ragged members, the per-class constants passed by value, the plan's layout and the
+// programmatic dependent launch.
 #pragma once
 
 #include <algorithm>
@@ -77,31 +76,28 @@ __device__ __forceinline__ void prefetch_tile_rows(int nrows, RowFn row) {
 int launch_forward(const ClassArgs& A, const TileSource& T, int ntiles, int kx_layout,
                    int grid_blocks, bool speculate, cudaStream_t st, cudaEvent_t marker);
 
+// Launches kernel<<<grid, threads, smem, st>>>(args...) as a programmatic dependent launch: its
+// blocks may start as the previous launch's blocks retire (they wait on the device,
+// griddepcontrol.wait, before reading what that launch writes).
+template <class... KArgs, class... Args>
+inline int launch_dependent(void (*kernel)(KArgs...), int grid, int threads, size_t smem,
+                            cudaStream_t st,
+                            Args... args) {
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  if (cudaLaunchKernelEx(&cfg, kernel, args...) != cudaSuccess) return SPD_ERR_CUDA;
+  return SPD_OK;
+}
+
 constexpr size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
-
-// M: any member record with in, C, il, kx, cls, S and table.
-template <int KX, class M>
-__device__ __forceinline__ void prepass_tile(const ClassArgs& A, const M& m, int c) {
-  const Consts& K = A.cls[m.cls].K;
-  if (c < m.il) m.table[c] = zonal_row(K.tyear, __ldg(m.in.sia + c), __ldg(m.in.coa + c));
-  const uint32_t bit = (c < m.C) ? prepass_column<KX>(K, m.in, c, m.C) : 0u;
-  or_level_set(bit, m.S);
-}
-
-template <class M>
-__device__ __forceinline__ void prepass_tiles(const ClassArgs& A, const M* __restrict__ members,
-                                              const Tile* __restrict__ tiles, int ntiles) {
-  for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-    const Tile tl = tiles[t];
-    const M& m = members[tl.member];
-    const int c = tl.col0 + threadIdx.x;
-    switch (m.kx) {  // uniform per block
-      case 16: prepass_tile<16>(A, m, c); break;
-      case 8: prepass_tile<8>(A, m, c); break;
-      default: prepass_tile<7>(A, m, c); break;
-    }
-  }
-}
 
 // Device plan layout: header, member records, tile list, level-set region, solar tables.  The
 // level-set region: 16 unused bytes, then nw words each of every member's T, an unused word and P

@@ -77,12 +77,21 @@ struct VjpMemberDev {
   ZonalRow* table;
 };
 
-// A field pointer of the member record, read where it is used: copied at the start, the record's
-// 28 pointers would hold 56 registers through the whole column.
+// Where an adjoint launch takes its members from: a plan's member table and tile list, or (when
+// `members` is null) the one member given by value, whose tile t covers columns t*kNT ..
+struct VjpSource {
+  const VjpMemberDev* members;
+  const Tile* tiles;
+  VjpMemberDev single;
+  int nmembers;
+};
+
+// A field pointer of the block's member record (in shared memory), read where it is used: held
+// from the start, the record's 28 pointers would take 56 registers through the whole column.
 template <class P>
-__device__ __forceinline__ P* field(P* const* at) {
+__device__ __forceinline__ P* load_field(P* const& at) {
   uint64_t v;
-  asm volatile("ld.global.nc.u64 %0, [%1];" : "=l"(v) : "l"(at));
+  asm volatile("ld.shared.u64 %0, [%1];" : "=l"(v) : "r"((uint32_t)__cvta_generic_to_shared(&at)));
   return reinterpret_cast<P*>(v);
 }
 
@@ -340,12 +349,11 @@ __device__ __forceinline__ void lw_rev_level(const ConstsD& CD, const LwCol& w, 
 // ---------------------------------------------------------------------------------------------
 // The column
 // ---------------------------------------------------------------------------------------------
-// Reverse pass of column c (clamped into the member by the caller, whose `valid` says whether to
-// store); adds the 12 parameter gradients to par.
+// Reverse pass of column c of member m (in shared memory), clamped into the member by the caller,
+// whose `valid` says whether to store; adds the 12 parameter gradients to par.
 template <int KX>
 __device__ __forceinline__ void column_vjp_smem(const ConstsD& CD, float* sm,
-                                                const VjpMemberDev* __restrict__ m,
-                                                const ZonalRow& z, uint32_t S, int c, int Ci,
+                                                const VjpMemberDev& m, int c, int Ci,
                                                 bool valid, float* par) {
   using spdvjp::fdiv;
   using spdvjp::frcp;
@@ -361,8 +369,8 @@ __device__ __forceinline__ void column_vjp_smem(const ConstsD& CD, float* sm,
   const Lv T = arr(V_T), Q = arr(V_Q), QS = arr(V_QS), TB = arr(V_TB), QB = arr(V_QB);
   const Lv S0 = arr(V_S0), S1 = arr(V_S1), S2 = arr(V_S2), S3 = arr(V_S3);
   const bool verify = (K.flags & SPD_FUSE_VERIFY) != 0;
-  const VjpColumn col{field(&m->in.geopotential) + c, field(&m->ct.temperature) + c,
-                      field(&m->ct.specific_humidity) + c, C};
+  const VjpColumn col{load_field(m.in.geopotential) + c, load_field(m.ct.temperature) + c,
+                      load_field(m.ct.specific_humidity) + c, C};
 
   // The rows that are first read further on start for L2 now, one row (128 bytes) per lane: the
   // two cotangents' levels, then the surface fields.
@@ -371,20 +379,22 @@ __device__ __forceinline__ void column_vjp_smem(const ConstsD& CD, float* sm,
     const int c0 = __shfl_sync(0xffffffffu, c, 0);  // the warp's first column
     const float* row = (lane < 16 ? col.ct_t : col.ct_q) - c + c0;
     if (level < KX) asm volatile("prefetch.global.L2 [%0];" ::"l"(row + level * C));
-    const float* const* fields = &m->in.alb0;  // alb0 .. phis0
-    if (lane < 9) asm volatile("prefetch.global.L2 [%0];" ::"l"(field(fields + lane) + c0));
+    if (lane < 9) {  // alb0 .. phis0
+      const float* f = load_field((&m.in.alb0)[lane]);
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(f + c0));
+    }
   }
 
   // ---- forward: humidity, convection, condensation, clouds ----------------------------------
   SurfaceIn s;
-  s.psa = __ldg(field(&m->in.normalized_surface_pressure) + c);
-  s.fmask = __ldg(field(&m->in.fmask) + c);
+  s.psa = __ldg(load_field(m.in.normalized_surface_pressure) + c);
+  s.fmask = __ldg(load_field(m.in.fmask) + c);
   const float psa = s.psa;
   ColScalars o;
   {
     float t[KX], q[KX], phi[KX], qs[KX], dt[KX], dq[KX];
-    const float* t_in = field(&m->in.temperature) + c;
-    const float* q_in = field(&m->in.specific_humidity) + c;
+    const float* t_in = load_field(m.in.temperature) + c;
+    const float* q_in = load_field(m.in.specific_humidity) + c;
 #pragma unroll
     for (int k = 0; k < KX; ++k) {
       t[k] = col.at(t_in, k);
@@ -413,8 +423,8 @@ __device__ __forceinline__ void column_vjp_smem(const ConstsD& CD, float* sm,
   spdvjp::SurfaceIn sf_in;
   float albsfc;
   {
-    const float snowc = __ldg(field(&m->in.snowc_am) + c), alb0 = __ldg(field(&m->in.alb0) + c);
-    sf_in.sice = __ldg(field(&m->in.sice_am) + c);
+    const float snowc = __ldg(load_field(m.in.snowc_am) + c), alb0 = __ldg(load_field(m.in.alb0) + c);
+    sf_in.sice = __ldg(load_field(m.in.sice_am) + c);
     sf_in.snowc = snowc;
     sf_in.alb0 = alb0;
     sf_in.fmask = fmask;
@@ -422,6 +432,23 @@ __device__ __forceinline__ void column_vjp_smem(const ConstsD& CD, float* sm,
     cc.alb_l = alb0 + cc.snowc * (p.albsn - alb0);
     const float alb_s = p.albsea + sf_in.sice * (p.albice - p.albsea);
     albsfc = alb_s + fmask * (cc.alb_l - alb_s);
+  }
+
+  // The level set and the solar rows are the pre-pass's: wait for it (this launch may start while
+  // it runs), then read them past L1.
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  const uint32_t S = __ldcg(load_field(m.S));
+  ZonalRow z;
+  {
+    const ZonalRow* zrow = load_field(m.table) + c % m.il;
+    const float4 a = __ldcg(reinterpret_cast<const float4*>(zrow));
+    const float2 b = __ldcg(reinterpret_cast<const float2*>(zrow) + 2);
+    z.fsol = a.x;
+    z.ozupp = a.y;
+    z.ozone = a.z;
+    z.zenit = a.w;
+    z.stratz = b.x;
+    z.sqrt_coa = b.y;
   }
 
   // ---- forward: shortwave (rs in S0, band-1 transmissivity in S1) ----------------------------
@@ -545,20 +572,20 @@ __device__ __forceinline__ void column_vjp_smem(const ConstsD& CD, float* sm,
   float sfc_q_b, sfc_phi_b, sfc_qs_b, u_b, v_b, rsds_b = 0.0f, rlds_b = 0.0f;
   {
     const float phiB = col.at(col.phi, B);
-    sf_in.sst = __ldg(field(&m->in.sea_surface_temperature) + c);
-    sf_in.stl = __ldg(field(&m->in.stl_am) + c);
-    sf_in.soilw = __ldg(field(&m->in.soilw_am) + c);
-    sf_in.orog = __ldg(field(&m->in.orog) + c);
-    sf_in.phis0 = __ldg(field(&m->in.phis0) + c);
-    const float ctu = col.at(field(&m->ct.u_wind) + c, B), ctv = col.at(field(&m->ct.v_wind) + c, B);
+    sf_in.sst = __ldg(load_field(m.in.sea_surface_temperature) + c);
+    sf_in.stl = __ldg(load_field(m.in.stl_am) + c);
+    sf_in.soilw = __ldg(load_field(m.in.soilw_am) + c);
+    sf_in.orog = __ldg(load_field(m.in.orog) + c);
+    sf_in.phis0 = __ldg(load_field(m.in.phis0) + c);
+    const float ctu = col.at(load_field(m.ct.u_wind) + c, B), ctv = col.at(load_field(m.ct.v_wind) + c, B);
     cc.psa = psa;
     cc.t[B] = T[B];
     cc.t[B - 1] = T[B - 1];
     cc.q[B] = Q[B];
     cc.qsat[B] = QS[B];
     cc.phi[B] = phiB;
-    cc.u = col.at(field(&m->in.u_wind) + c, B);
-    cc.v = col.at(field(&m->in.v_wind) + c, B);
+    cc.u = col.at(load_field(m.in.u_wind) + c, B);
+    cc.v = col.at(load_field(m.in.v_wind) + c, B);
     cc.rsds = rsds;
     cc.rlds = rlds;
     const spdvjp::Ctx x{&vg, &p, K.flags, K.model_step, S};
@@ -591,7 +618,7 @@ __device__ __forceinline__ void column_vjp_smem(const ConstsD& CD, float* sm,
                                          D.pexp)
               : 0.0f;
       const float dts = K.dt_seconds;
-      const float* q_in = field(&m->in.specific_humidity) + c;
+      const float* q_in = load_field(m.in.specific_humidity) + c;
       float pend = 0.0f, rh_k = 0.0f;
 #pragma unroll 2
       for (int k = 0; k < KX; ++k) {
@@ -1324,10 +1351,10 @@ __device__ __forceinline__ void column_vjp_smem(const ConstsD& CD, float* sm,
     const float rdt = K.dt_seconds;
     // plain loads, each level's before the level above it is stored: a gradient may share its
     // buffer with an input or a cotangent
-    const float* q_in = field(&m->in.specific_humidity) + c;
-    float *gt = field(&m->gr.temperature) + c, *gq = field(&m->gr.specific_humidity) + c,
-          *gp = field(&m->gr.geopotential) + c, *gu = field(&m->gr.u_wind) + c,
-          *gv = field(&m->gr.v_wind) + c;
+    const float* q_in = load_field(m.in.specific_humidity) + c;
+    float *gt = load_field(m.gr.temperature) + c, *gq = load_field(m.gr.specific_humidity) + c,
+          *gp = load_field(m.gr.geopotential) + c, *gu = load_field(m.gr.u_wind) + c,
+          *gv = load_field(m.gr.v_wind) + c;
     float cq_n = col.ct_q[0], ct_n = col.ct_t[0], qi_n = verify ? q_in[0] : 0.0f;
 #pragma unroll 2
     for (int k = 0; k < KX; ++k) {
@@ -1387,7 +1414,7 @@ __device__ __forceinline__ void column_vjp_smem(const ConstsD& CD, float* sm,
     if (valid) {
       gu[B * C] = u_b;
       gv[B * C] = v_b;
-      field(&m->gr.normalized_surface_pressure)[c] = psa_b;
+      load_field(m.gr.normalized_surface_pressure)[c] = psa_b;
     }
   }
 }
