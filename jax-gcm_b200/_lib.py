@@ -205,6 +205,37 @@ def load():
     return _lib
 
 
+_calls = None
+
+
+def calls():
+    """The extension module that hands torch tensors to the library (``csrc/torch_calls.cpp``,
+    built by ``build.py`` for the installed torch).  Raises SpeedyLibraryError when it is
+    missing."""
+    global _calls
+    if _calls is None:
+        import importlib.machinery
+        import importlib.util
+
+        import torch
+        path = os.path.join(HERE, "_calls.torch" + torch.__version__.split("+")[0] + ".so")
+        if not os.path.exists(path):
+            raise SpeedyLibraryError(
+                f"{path} is missing: build it with `python -c 'import __graft_entry__ as g; "
+                "g.build()'`")
+        lib = load()
+        with _lock:
+            if _calls is None:
+                loader = importlib.machinery.ExtensionFileLoader("_calls", path)
+                mod = importlib.util.module_from_spec(
+                    importlib.util.spec_from_loader("_calls", loader))
+                loader.exec_module(mod)
+                mod.bind(*(C.cast(f, C.c_void_p).value
+                           for f in (lib.spd_fwd_marked, lib.spd_vjp, lib.spd_held_suarez)))
+                _calls = mod
+    return _calls
+
+
 def check(rc, what="spd call"):
     if rc != 0:
         msg = load().spd_status_string(rc).decode()

@@ -18,8 +18,7 @@ import numpy as np
 import torch
 
 from . import _lib
-from .physics import (Parameters, PhysicsState, PhysicsTendency, SpeedyPhysics,
-                      current_raw_stream)
+from .physics import Parameters, PhysicsState, PhysicsTendency, SpeedyPhysics
 
 DIFF_PARAMS = [("convection", "psmin"), ("convection", "trcnv"), ("convection", "rhil"),
                ("convection", "rhbl"), ("convection", "entmax"), ("convection", "smf"),
@@ -39,53 +38,22 @@ def _scratch(nbytes, device):
     return buf
 
 
-def _input_struct(state, forcing, geometry):
-    f2 = forcing
-    t = dict(u_wind=state.u_wind, v_wind=state.v_wind, temperature=state.temperature,
-             specific_humidity=state.specific_humidity, geopotential=state.geopotential,
-             normalized_surface_pressure=state.normalized_surface_pressure, alb0=f2.alb0,
-             sice_am=f2.sice_am, snowc_am=f2.snowc_am, soilw_am=f2.soilw_am, stl_am=f2.stl_am,
-             sea_surface_temperature=f2.sea_surface_temperature, fmask=geometry.fmask,
-             orog=geometry.orog, phis0=geometry.phis0, sia=geometry.sia, coa=geometry.coa)
-    dev = state.temperature.device
-    didx = state.temperature.get_device()
-    ptrs = []
-    for k in _lib.INPUT_FIELDS:
-        v = t[k]
-        if v.dtype is not torch.float32 or not v.is_contiguous() or v.get_device() != didx:
-            v = t[k] = v.to(device=dev, dtype=torch.float32).contiguous()
-        ptrs.append(v.data_ptr())
-    return _lib.Inputs(*ptrs), t
-
-
 def vjp(physics: SpeedyPhysics, state: PhysicsState, forcing, geometry, date,
         cotangent: PhysicsTendency):
     """(PhysicsState of gradients, tensor[12] of parameter gradients) for the cotangent."""
     lib = _lib.load()
+    calls = _lib.calls()
     dev = state.temperature.device
     _lib.preload(dev.index if dev.index is not None else torch.cuda.current_device())
     f2 = forcing.day_slice(date.model_day())
-    inp, keep = _input_struct(state, f2, geometry)
-    ct = {k: getattr(cotangent, k).to(device=dev, dtype=torch.float32).contiguous()
-          for k in ("u_wind", "v_wind", "temperature", "specific_humidity")}
-    cts = _lib.Cotangents(**{k: v.data_ptr() for k, v in ct.items()})
-    e = lambda ref: torch.empty_like(ref)
-    g = dict(u_wind=e(state.u_wind), v_wind=e(state.v_wind), temperature=e(state.temperature),
-             specific_humidity=e(state.specific_humidity), geopotential=e(state.geopotential),
-             normalized_surface_pressure=e(state.normalized_surface_pressure),
-             params=torch.empty(12, dtype=torch.float32, device=dev))
-    grads = _lib.Grads(**{k: v.data_ptr() for k, v in g.items()})
     desc = physics.desc(geometry, date, forcing.lfluxland)
     n = lib.spd_vjp_scratch_bytes(C.byref(desc))
     sc = _scratch(n, dev)
-    stream = current_raw_stream(state.temperature.get_device())
-    rc = lib.spd_vjp(C.byref(desc), C.byref(geometry.vgrid()), C.byref(physics._pstruct),
-                     C.byref(inp), C.byref(cts), C.byref(grads), C.c_void_p(sc.data_ptr()), n,
-                     C.c_void_p(stream))
+    rc, g = calls.vjp(state, f2, geometry, cotangent, C.addressof(desc),
+                      C.addressof(geometry.vgrid()), C.addressof(physics._pstruct), sc.data_ptr(),
+                      n)
     _lib.check(rc, "spd_vjp")
-    gs = PhysicsState(g["u_wind"], g["v_wind"], g["temperature"], g["specific_humidity"],
-                      g["geopotential"], g["normalized_surface_pressure"])
-    return gs, g["params"]
+    return PhysicsState(*g[:6]), g[6]
 
 
 # ---------------------------------------------------------------------------------------------

@@ -1,7 +1,9 @@
 """Builds ``libspeedy_b200.so`` in-tree with nvcc for sm_100a (no JIT cache, no torch ABI).
 
 Each translation unit is compiled to an object in parallel, then linked into one shared
-library; objects go to ``jax-gcm_b200/_build/`` (not committed).
+library; objects go to ``jax-gcm_b200/_build/`` (not committed).  Beside it, g++ builds the
+extension module through which the Python calls hand torch tensors to the library
+(``csrc/torch_calls.cpp``), against the installed torch and named by its version.
 """
 from __future__ import annotations
 
@@ -19,6 +21,7 @@ HEADERS = ["csrc/speedy_column.cuh", "csrc/speedy_column_smem.cuh", "csrc/speedy
            "csrc/speedy_generic.h", "csrc/speedy_vjp.h", "csrc/speedy_vjp_smem.cuh",
            "csrc/speedy_pk.cuh",
            "../include/speedy_b200.h"]
+CALLS_SOURCE = "csrc/torch_calls.cpp"
 OUT = os.path.join(HERE, "libspeedy_b200.so")
 OBJ_DIR = os.path.join(HERE, "_build")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
@@ -57,6 +60,35 @@ def compile_command(src, verbose=False):
     return cmd, obj
 
 
+def calls_path():
+    import torch
+    return os.path.join(HERE, "_calls.torch" + torch.__version__.split("+")[0] + ".so")
+
+
+def calls_command():
+    """The compile command of the torch extension module."""
+    import sysconfig
+
+    import torch
+    lib = os.path.join(os.path.dirname(torch.__file__), "lib")
+    inc = os.path.join(os.path.dirname(torch.__file__), "include")
+    cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    return [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-shared", "-fPIC",
+            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+            "-I" + os.path.join(ROOT, "include"), "-I" + inc,
+            "-I" + os.path.join(inc, "torch", "csrc", "api", "include"),
+            "-I" + sysconfig.get_paths()["include"], "-I" + os.path.join(cuda, "include"),
+            os.path.join(HERE, CALLS_SOURCE), "-o", calls_path(), "-L" + lib, "-ltorch_python",
+            "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda"]
+
+
+def needs_calls():
+    out = calls_path()
+    deps = [CALLS_SOURCE, "../include/speedy_b200.h", os.path.basename(__file__)]
+    return not os.path.exists(out) or any(
+        os.path.getmtime(os.path.join(HERE, d)) > os.path.getmtime(out) for d in deps)
+
+
 def needs_build():
     if not os.path.exists(OUT):
         return True
@@ -66,6 +98,11 @@ def needs_build():
 
 
 def build(force=False, verbose=False):
+    if force or needs_calls():
+        res = subprocess.run(calls_command(), capture_output=True, text=True)
+        if res.returncode != 0:
+            sys.stderr.write(res.stdout + res.stderr)
+            raise RuntimeError("g++ failed: " + " ".join(calls_command()))
     if not force and not needs_build():
         return OUT
     os.makedirs(OBJ_DIR, exist_ok=True)

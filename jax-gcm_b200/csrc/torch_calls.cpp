@@ -1,0 +1,264 @@
+// torch_calls.cpp -- the plain calls on torch tensors: gathers the field pointers, allocates the
+// results and calls the C ABI, for physics.py, adjoint.py and held_suarez.py.
+//
+// A small call is bound by the host: through ctypes a T21 call with its diagnostics took 91 us, of
+// which the device works 17 (21 torch.empty calls of 2.4 us each, 38 pointers, the structures).
+// Through this module it takes 38 us (T85 with 16 levels 45 -> 25, a T42 VJP with 8 levels 44 ->
+// 31, a 361 x 181 Held-Suarez call 27 -> 16); 21 of the 38 are the 21 result tensors.  It does the
+// same in one call: 17 attribute reads and checks, one allocation per result
+// through torch's allocator, and the library call with the interpreter's lock released.  Nothing is
+// kept between calls.  The library's entry points come in as addresses (bind), so that this module
+// does not depend on which build of the library is loaded.
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/utils/pybind.h>
+
+#include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDAStream.h>
+
+#include <array>
+
+#include "speedy_b200.h"
+
+namespace {
+
+decltype(&spd_fwd_marked) g_fwd = nullptr;
+decltype(&spd_vjp) g_vjp = nullptr;
+decltype(&spd_held_suarez) g_hs = nullptr;
+
+enum Owner { kState, kForcing, kGeometry };
+struct Name {
+  const char* text;
+  Owner owner;
+  PyObject* str;
+};
+// spd_inputs_t in order.
+Name g_inputs[] = {{"u_wind", kState, nullptr}, {"v_wind", kState, nullptr},
+                   {"temperature", kState, nullptr}, {"specific_humidity", kState, nullptr},
+                   {"geopotential", kState, nullptr},
+                   {"normalized_surface_pressure", kState, nullptr}, {"alb0", kForcing, nullptr},
+                   {"sice_am", kForcing, nullptr}, {"snowc_am", kForcing, nullptr},
+                   {"soilw_am", kForcing, nullptr}, {"stl_am", kForcing, nullptr},
+                   {"sea_surface_temperature", kForcing, nullptr}, {"fmask", kGeometry, nullptr},
+                   {"orog", kGeometry, nullptr}, {"phis0", kGeometry, nullptr},
+                   {"sia", kGeometry, nullptr}, {"coa", kGeometry, nullptr}};
+constexpr int kInputs = sizeof(g_inputs) / sizeof(g_inputs[0]);
+static_assert(kInputs * sizeof(void*) == sizeof(spd_inputs_t), "one pointer per input field");
+constexpr int kOutputs = sizeof(spd_outputs_t) / sizeof(void*);
+constexpr int kLevelOutputs = 4, kFloatOutputs = 19, kPlainOutputs = 6;
+
+at::Tensor attribute(PyObject* obj, PyObject* name) {
+  PyObject* v = PyObject_GetAttr(obj, name);
+  if (!v) throw python_error();
+  const bool is = THPVariable_Check(v);
+  at::Tensor t = is ? THPVariable_Unpack(v) : at::Tensor();
+  Py_DECREF(v);
+  TORCH_CHECK_TYPE(is, PyUnicode_AsUTF8(name), " must be a tensor");
+  return t;
+}
+
+// `t` as contiguous float32 on `device`; itself where it is that already.
+at::Tensor as_input(at::Tensor t, c10::Device device) {
+  if (t.scalar_type() != at::kFloat || !t.is_contiguous() || t.device() != device)
+    return t.to(device, at::kFloat).contiguous();
+  return t;
+}
+
+c10::Device device_of(PyObject* state, int temperature = 2) {
+  return attribute(state, g_inputs[temperature].str).device();
+}
+
+struct Fields {
+  std::array<at::Tensor, kInputs> t;  // keeps converted copies until the call is enqueued
+  spd_inputs_t in;
+};
+
+Fields fields(PyObject* state, PyObject* forcing, PyObject* geometry, c10::Device device) {
+  PyObject* const owners[] = {state, forcing, geometry};
+  Fields f;
+  const float** p = reinterpret_cast<const float**>(&f.in);
+  for (int i = 0; i < kInputs; ++i) {
+    f.t[i] = as_input(attribute(owners[g_inputs[i].owner], g_inputs[i].str), device);
+    p[i] = static_cast<const float*>(f.t[i].const_data_ptr());
+  }
+  return f;
+}
+
+// A result tensor, from torch's caching allocator.
+at::Tensor empty(at::IntArrayRef shape, c10::Device device, at::ScalarType type = at::kFloat) {
+  return at::detail::empty_cuda(shape, type, device, std::nullopt);
+}
+
+template <class T>
+T* address(PyObject* v) {
+  void* p = PyLong_AsVoidPtr(v);
+  if (!p && PyErr_Occurred()) throw python_error();
+  return static_cast<T*>(p);
+}
+
+void* stream_of(c10::Device device) {
+  return c10::cuda::getCurrentCUDAStream(device.index()).stream();
+}
+
+PyObject* result(int rc, const at::Tensor* t, int n) {
+  PyObject* list = PyList_New(n);
+  if (!list) throw python_error();
+  for (int i = 0; i < n; ++i) {
+    PyObject* v = t[i].defined() ? THPVariable_Wrap(t[i]) : (Py_INCREF(Py_None), Py_None);
+    PyList_SET_ITEM(list, i, v);
+  }
+  return Py_BuildValue("(iN)", rc, list);
+}
+
+void expect(Py_ssize_t have, Py_ssize_t want) {
+  TORCH_CHECK_TYPE(have == want, "expected ", want, " arguments, got ", have);
+}
+
+// fwd(state, forcing, geometry, out, diagnostics, desc, vgrid, params, scratch, scratch_bytes,
+//     event) -> (status, [tensor or None per spd_outputs_t field])
+// out: None, or a list of tensors or None in spd_outputs_t's order.
+PyObject* fwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  expect(n, 11);
+  const auto* desc = address<const spd_desc_t>(a[5]);
+  const c10::Device device = device_of(a[0]);
+  Fields f = fields(a[0], a[1], a[2], device);
+  std::array<at::Tensor, kOutputs> t;
+  spd_outputs_t out{};
+  void** p = reinterpret_cast<void**>(&out);
+  if (a[3] == Py_None) {
+    const int64_t level[] = {desc->kx, desc->ix, desc->il}, surface[] = {desc->ix, desc->il};
+    const int count = PyObject_IsTrue(a[4]) == 1 ? kOutputs : kPlainOutputs;
+    for (int i = 0; i < count; ++i) {
+      t[i] = i < kLevelOutputs ? empty(level, device)
+                               : empty(surface, device, i < kFloatOutputs ? at::kFloat : at::kInt);
+      p[i] = t[i].data_ptr();
+    }
+  } else {
+    TORCH_CHECK_TYPE(PyList_Check(a[3]) && PyList_GET_SIZE(a[3]) == kOutputs, "out is a list");
+    for (int i = 0; i < kOutputs; ++i) {
+      PyObject* v = PyList_GET_ITEM(a[3], i);
+      if (v == Py_None) continue;
+      TORCH_CHECK_TYPE(THPVariable_Check(v), "out holds tensors");
+      t[i] = THPVariable_Unpack(v);
+      p[i] = t[i].data_ptr();
+    }
+  }
+  void* stream = stream_of(device);
+  const auto* vgrid = address<const spd_vgrid_t>(a[6]);
+  const auto* params = address<const spd_params_t>(a[7]);
+  void* scratch = address<void>(a[8]);
+  const size_t bytes = PyLong_AsSize_t(a[9]);
+  void* event = address<void>(a[10]);
+  int rc;
+  {
+    pybind11::gil_scoped_release release;
+    rc = g_fwd(desc, vgrid, params, &f.in, &out, scratch, bytes, stream, event);
+  }
+  return result(rc, t.data(), kOutputs);
+  END_HANDLE_TH_ERRORS
+}
+
+// vjp(state, forcing, geometry, cotangent, desc, vgrid, params, scratch, scratch_bytes)
+//   -> (status, [u, v, T, q, phi, psa, params gradients])
+PyObject* vjp(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  expect(n, 9);
+  const c10::Device device = device_of(a[0]);
+  TORCH_CHECK(device.is_cuda(), "the adjoint runs on CUDA tensors only (no CPU path)");
+  Fields f = fields(a[0], a[1], a[2], device);
+  std::array<at::Tensor, 4> ct;
+  spd_cotangents_t cot;
+  const float** pc = reinterpret_cast<const float**>(&cot);
+  for (int i = 0; i < 4; ++i) {
+    ct[i] = as_input(attribute(a[3], g_inputs[i].str), device);
+    pc[i] = static_cast<const float*>(ct[i].const_data_ptr());
+  }
+  std::array<at::Tensor, 7> g;
+  spd_grads_t grads;
+  float** pg = reinterpret_cast<float**>(&grads);
+  for (int i = 0; i < 7; ++i) {
+    g[i] = i < 6 ? empty(f.t[i].sizes(), device) : empty({SPD_NUM_DIFF_PARAMS}, device);
+    pg[i] = static_cast<float*>(g[i].data_ptr());
+  }
+  void* stream = stream_of(device);
+  const auto* desc = address<const spd_desc_t>(a[4]);
+  const auto* vgrid = address<const spd_vgrid_t>(a[5]);
+  const auto* params = address<const spd_params_t>(a[6]);
+  void* scratch = address<void>(a[7]);
+  const size_t bytes = PyLong_AsSize_t(a[8]);
+  int rc;
+  {
+    pybind11::gil_scoped_release release;
+    rc = g_vjp(desc, vgrid, params, &f.in, &cot, &grads, scratch, bytes, stream);
+  }
+  return result(rc, g.data(), 7);
+  END_HANDLE_TH_ERRORS
+}
+
+// held_suarez(state, table, out, desc) -> (status, [du, dv, dT, dq]); out: None or four tensors.
+PyObject* held_suarez(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  expect(n, 4);
+  const c10::Device device = device_of(a[0]);
+  const int which[] = {0, 1, 2, 5};  // u, v, T, psa
+  std::array<at::Tensor, 4> in, out;
+  for (int i = 0; i < 4; ++i) in[i] = as_input(attribute(a[0], g_inputs[which[i]].str), device);
+  TORCH_CHECK_TYPE(THPVariable_Check(a[1]), "the latitude table is a tensor");
+  const at::Tensor& table = THPVariable_Unpack(a[1]);
+  for (int i = 0; i < 4; ++i) {
+    if (a[2] == Py_None) {
+      out[i] = empty(in[2].sizes(), device);
+    } else {
+      TORCH_CHECK_TYPE(PyList_Check(a[2]) && PyList_GET_SIZE(a[2]) == 4, "out is a list of four");
+      PyObject* v = PyList_GET_ITEM(a[2], i);
+      TORCH_CHECK_TYPE(THPVariable_Check(v), "out holds tensors");
+      out[i] = THPVariable_Unpack(v);
+    }
+  }
+  const auto* desc = address<const spd_hs_desc_t>(a[3]);
+  void* stream = stream_of(device);
+  auto p = [](const at::Tensor& t) { return static_cast<const float*>(t.const_data_ptr()); };
+  auto w = [](const at::Tensor& t) { return static_cast<float*>(t.data_ptr()); };
+  const float* lat = p(table);
+  const float *u = p(in[0]), *v = p(in[1]), *t = p(in[2]), *psa = p(in[3]);
+  float *du = w(out[0]), *dv = w(out[1]), *dt = w(out[2]), *dq = w(out[3]);
+  int rc;
+  {
+    pybind11::gil_scoped_release release;
+    rc = g_hs(desc, lat, u, v, t, psa, du, dv, dt, dq, stream);
+  }
+  return result(rc, out.data(), 4);
+  END_HANDLE_TH_ERRORS
+}
+
+// bind(spd_fwd_marked, spd_vjp, spd_held_suarez): the library's entry points, as addresses.
+PyObject* bind(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  expect(n, 3);
+  g_fwd = reinterpret_cast<decltype(g_fwd)>(address<void>(a[0]));
+  g_vjp = reinterpret_cast<decltype(g_vjp)>(address<void>(a[1]));
+  g_hs = reinterpret_cast<decltype(g_hs)>(address<void>(a[2]));
+  Py_RETURN_NONE;
+  END_HANDLE_TH_ERRORS
+}
+
+template <PyObject* (*F)(PyObject*, PyObject* const*, Py_ssize_t)>
+PyMethodDef method(const char* name) {
+  return {name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(F)), METH_FASTCALL,
+          nullptr};
+}
+
+PyMethodDef g_methods[] = {method<fwd>("fwd"), method<vjp>("vjp"),
+                           method<held_suarez>("held_suarez"), method<bind>("bind"),
+                           {nullptr, nullptr, 0, nullptr}};
+PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "_calls", nullptr, -1, g_methods,
+                        nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__calls() {
+  for (Name& n : g_inputs)
+    if (!(n.str = PyUnicode_InternFromString(n.text))) return nullptr;
+  return PyModule_Create(&g_module);
+}

@@ -20,6 +20,7 @@ from . import _lib
 from .physics import Geometry, Physics, PhysicsState, PhysicsTendency
 
 DAY = 86400.0
+OUT_FIELDS = ("u_wind", "v_wind", "temperature", "specific_humidity")
 
 
 class HeldSuarezPhysics(Physics):
@@ -60,7 +61,7 @@ class HeldSuarezPhysics(Physics):
         u_wind, v_wind, temperature, specific_humidity tensors."""
         if geometry is None:
             raise ValueError("HeldSuarezPhysics needs the Geometry (level centres, latitudes)")
-        lib = _lib.load()
+        calls = _lib.calls()
         t = state.temperature
         if t.device.type != "cuda":
             raise RuntimeError("HeldSuarezPhysics runs on CUDA tensors only (no CPU path)")
@@ -69,18 +70,9 @@ class HeldSuarezPhysics(Physics):
                              f"{tuple(geometry.nodal_shape)}")
         dev = t.device
         _lib.preload(dev.index if dev.index is not None else torch.cuda.current_device())
-        f = lambda x: x.to(device=dev, dtype=torch.float32).contiguous()
-        u, v, tt, ps = (f(state.u_wind), f(state.v_wind), f(t),
-                        f(state.normalized_surface_pressure))
-        if out is None:
-            out = {k: torch.empty_like(tt) for k in ("u_wind", "v_wind", "temperature",
-                                                      "specific_humidity")}
-        tab = self._lat_table(geometry, dev)
-        p = lambda x: C.c_void_p(x.data_ptr())
-        stream = torch.cuda.current_stream(dev).cuda_stream
-        rc = lib.spd_held_suarez(C.byref(self._desc(geometry)), p(tab), p(u), p(v), p(tt), p(ps),
-                                 p(out["u_wind"]), p(out["v_wind"]), p(out["temperature"]),
-                                 p(out["specific_humidity"]), C.c_void_p(stream))
+        desc = self._desc(geometry)
+        rc, o = calls.held_suarez(state, self._lat_table(geometry, dev),
+                                  None if out is None else [out[k] for k in OUT_FIELDS],
+                                  C.addressof(desc))
         _lib.check(rc, "spd_held_suarez")
-        return PhysicsTendency(out["u_wind"], out["v_wind"], out["temperature"],
-                               out["specific_humidity"]), None
+        return PhysicsTendency(*o), None

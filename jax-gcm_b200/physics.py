@@ -427,17 +427,6 @@ def physics_data_from_diagnostics(d):
     )
 
 
-def _ptr(t):
-    return C.c_void_p(t.data_ptr())
-
-
-def current_raw_stream(device_index):
-    """The current CUDA stream of a device as a raw handle (torch's own fast path where it has
-    one; torch.cuda.current_stream otherwise)."""
-    f = getattr(torch._C, "_cuda_getCurrentRawStream", None)
-    return f(device_index) if f is not None else torch.cuda.current_stream(device_index).cuda_stream
-
-
 class SpeedyPhysics(Physics):
     """SPEEDY physics on the B200 (speedy_physics.py:34-132).
 
@@ -514,57 +503,29 @@ class SpeedyPhysics(Physics):
         DiagnosticsCollector, jcm/model.py:46-64; scale by 1/steps once at the end)."""
         if accumulate and out is None:
             raise ValueError("accumulate=True adds into `out`: pass the running sums")
-        lib = _lib.load()
-        kx, ix, il = geometry.nodal_shape
+        calls = _lib.calls()
         t = state.temperature
-        if tuple(t.shape) != (kx, ix, il):
-            raise ValueError(f"state shape {tuple(t.shape)} does not match geometry {(kx, ix, il)}")
+        if t.shape != tuple(geometry.nodal_shape):
+            raise ValueError(f"state shape {tuple(t.shape)} does not match geometry "
+                             f"{tuple(geometry.nodal_shape)}")
         if not t.is_cuda:
             raise RuntimeError("SpeedyPhysics runs on CUDA tensors only (no CPU path)")
-        dev = t.device
-        didx = t.get_device()
-        _lib.preload(didx)
+        _lib.preload(t.get_device())
         if self._day[0] != date.tyear:
             self._day = (date.tyear, date.model_day())
         f2 = forcing.day_slice(self._day[1])
-        tensors = dict(u_wind=state.u_wind, v_wind=state.v_wind, temperature=state.temperature,
-                       specific_humidity=state.specific_humidity,
-                       geopotential=state.geopotential,
-                       normalized_surface_pressure=state.normalized_surface_pressure,
-                       alb0=f2.alb0, sice_am=f2.sice_am, snowc_am=f2.snowc_am,
-                       soilw_am=f2.soilw_am, stl_am=f2.stl_am,
-                       sea_surface_temperature=f2.sea_surface_temperature, fmask=geometry.fmask,
-                       orog=geometry.orog, phis0=geometry.phis0, sia=geometry.sia,
-                       coa=geometry.coa)
-        ptrs = []
-        for k in _lib.INPUT_FIELDS:
-            v = tensors[k]
-            if v.dtype is not torch.float32 or not v.is_contiguous() or v.get_device() != didx:
-                v = tensors[k] = v.to(device=dev, dtype=torch.float32).contiguous()
-            ptrs.append(v.data_ptr())
-        if out is None:
-            e3 = lambda: torch.empty((kx, ix, il), dtype=torch.float32, device=dev)
-            e2 = lambda: torch.empty((ix, il), dtype=torch.float32, device=dev)
-            out = dict(u_wind=e3(), v_wind=e3(), temperature=e3(), specific_humidity=e3(),
-                       precnv=e2(), precls=e2())
-            if self.diagnostics:
-                for n in DIAG_2D:
-                    out[n] = e2()
-                out["iptop"] = torch.empty((ix, il), dtype=torch.int32, device=dev)
-                out["icltop"] = torch.empty((ix, il), dtype=torch.int32, device=dev)
-        inp = _lib.Inputs(*ptrs)
-        outs = _lib.Outputs(*[out[k].data_ptr() if k in out else None
-                              for k in _lib.OUTPUT_FIELDS])
         desc = self.desc(geometry, date, forcing.lfluxland)
         if accumulate:
             desc.flags |= _lib.SPD_ACCUMULATE_DIAGNOSTICS
-        scratch = self._scratch_for(desc, dev)
-        stream = current_raw_stream(didx)
-        ev = C.c_void_p(marker.cuda_event) if marker is not None else None
-        rc = lib.spd_fwd_marked(C.byref(desc), C.byref(geometry.vgrid()), C.byref(self._pstruct),
-                                C.byref(inp), C.byref(outs), _ptr(scratch), scratch.numel(),
-                                C.c_void_p(stream), ev)
+        scratch = self._scratch_for(desc, t.device)
+        given = None if out is None else [out.get(k) for k in _lib.OUTPUT_FIELDS]
+        rc, outs = calls.fwd(state, f2, geometry, given, self.diagnostics, C.addressof(desc),
+                             C.addressof(geometry.vgrid()), C.addressof(self._pstruct),
+                             scratch.data_ptr(), scratch.numel(),
+                             0 if marker is None else marker.cuda_event)
         _lib.check(rc, "spd_fwd")
+        if out is None:
+            out = dict(zip(_lib.OUTPUT_FIELDS, outs))
         tend = PhysicsTendency(out["u_wind"], out["v_wind"], out["temperature"],
                                out["specific_humidity"])
         return tend, physics_data_from_diagnostics(out)

@@ -89,7 +89,8 @@ def test_gradients_may_overwrite_the_cotangents(pkg):
     buf = {n: t.clone() for n, t in ct.items()}
     phi, psa = torch.empty_like(state.geopotential), torch.empty(ix, il, device="cuda")
     par = torch.empty(12, device="cuda")
-    inp, keep = pkg.adjoint._input_struct(state, forcing, geom)
+    owner = lambda n: next(o for o in (state, forcing, geom) if hasattr(o, n))
+    inp = L.Inputs(*(getattr(owner(n), n).data_ptr() for n in L.INPUT_FIELDS))
     cts = L.Cotangents(**{n: t.data_ptr() for n, t in buf.items()})
     grads = L.Grads(**{n: t.data_ptr() for n, t in buf.items()}, geopotential=phi.data_ptr(),
                     normalized_surface_pressure=psa.data_ptr(), params=par.data_ptr())
