@@ -391,6 +391,7 @@ __device__ __forceinline__ void column_vjp_smem(const ConstsD& CD, float* sm,
   s.fmask = __ldg(load_field(m.in.fmask) + c);
   const float psa = s.psa;
   ColScalars o;
+  uint32_t neg = 0u;  // levels whose humidity verify_state clamped
   {
     float t[KX], q[KX], phi[KX], qs[KX], dt[KX], dq[KX];
     const float* t_in = load_field(m.in.temperature) + c;
@@ -399,6 +400,7 @@ __device__ __forceinline__ void column_vjp_smem(const ConstsD& CD, float* sm,
     for (int k = 0; k < KX; ++k) {
       t[k] = col.at(t_in, k);
       const float qk = col.at(q_in, k);
+      if (verify && qk < 0.0f) neg |= 1u << k;
       q[k] = (verify && qk < 0.0f) ? 0.0f : qk;
       phi[k] = col.at(col.phi, k);
     }
@@ -641,8 +643,15 @@ __device__ __forceinline__ void column_vjp_smem(const ConstsD& CD, float* sm,
           dq = dq + 0.0f;
         }
         if (oro) dq = dq + fdiv(qcorh * D.qcorv[k], dts);
-        if (!(col.at(q_in, k) + dts * dq >= 0.0f)) limited |= 1u << k;
+        TB[k] = dq;
       }
+      // the humidity as given, read again where it was clamped, all levels' loads first
+      float qi[KX];
+#pragma unroll
+      for (int k = 0; k < KX; ++k) qi[k] = ((neg >> k) & 1u) ? col.at(q_in, k) : Q[k];
+#pragma unroll
+      for (int k = 0; k < KX; ++k)
+        if (!(qi[k] + dts * TB[k] >= 0.0f)) limited |= 1u << k;
     }
     // the upward pass starts from the surface's fluxes
     float2 f01, f23;
@@ -1351,19 +1360,16 @@ __device__ __forceinline__ void column_vjp_smem(const ConstsD& CD, float* sm,
     const float rdt = K.dt_seconds;
     // plain loads, each level's before the level above it is stored: a gradient may share its
     // buffer with an input or a cotangent
-    const float* q_in = load_field(m.in.specific_humidity) + c;
     float *gt = load_field(m.gr.temperature) + c, *gq = load_field(m.gr.specific_humidity) + c,
           *gp = load_field(m.gr.geopotential) + c, *gu = load_field(m.gr.u_wind) + c,
           *gv = load_field(m.gr.v_wind) + c;
-    float cq_n = col.ct_q[0], ct_n = col.ct_t[0], qi_n = verify ? q_in[0] : 0.0f;
+    float cq_n = col.ct_q[0], ct_n = col.ct_t[0];
 #pragma unroll 2
     for (int k = 0; k < KX; ++k) {
       const float ctq = cq_n * K.q_tend_scale, ctt_k = ct_n;
-      const bool negative = verify && qi_n < 0.0f;
       const size_t in1 = (k < B ? k + 1 : B) * C;
       cq_n = col.ct_q[in1];
       ct_n = col.ct_t[in1];
-      if (verify) qi_n = q_in[in1];
       const float t = T[k], q = Q[k], qs = QS[k];
       float qs_b = XB[k], q_b = QB[k];
       const bool lim = (limited >> k) & 1u;
@@ -1398,7 +1404,7 @@ __device__ __forceinline__ void column_vjp_smem(const ConstsD& CD, float* sm,
       const float tb = TB[k] + x * fdiv(a, den * den);
       if (valid) {
         const size_t i = k * C;
-        const float qk = negative ? 0.0f : q_b;
+        const float qk = ((neg >> k) & 1u) ? 0.0f : q_b;
         __stcs(gt + i, tb);
         __stcs(gq + i, qk + (lim ? -fdiv(ctq, rdt) : 0.0f));
         __stcs(gp + i, PB[k]);
