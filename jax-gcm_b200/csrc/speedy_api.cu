@@ -135,7 +135,8 @@ int dispatch_fwd(const ConstsD& CD, int kx, const spd_inputs_t& in, const spd_ou
   const bool speculate =
       (CD.K.flags & (SPD_ACCUMULATE_DIAGNOSTICS | SPD_NO_SPECULATION)) == 0;
   const int ntiles = (CD.K.C + kNT - 1) / kNT;
-  return launch_forward(A, T, ntiles, kx, SPD_GRID_PER_TILE, speculate, st, marker);
+  return launch_forward(A, T, ntiles, kx, SPD_GRID_PER_TILE, speculate,
+                        (CD.K.flags & SPD_FUSE_VERIFY) != 0, st, marker);
 }
 
 int preload_ensemble();

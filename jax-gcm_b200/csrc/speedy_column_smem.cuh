@@ -405,10 +405,11 @@ __device__ __forceinline__ void column_first(const ConstsD& C, const float (&T)[
 }
 
 // Second half: shortwave, longwave, surface fluxes and vertical diffusion, from the state, qsat
-// and tendency accumulators in shared memory and the first half's results in o.
-template <int KX>
+// and tendency accumulators in shared memory and the first half's results in o.  work_free() is
+// called once the work array W is no longer needed, before the vertical diffusion.
+template <int KX, class F>
 __device__ void column_second(const ConstsD& C, float* sm, const SurfaceIn& s, const ZonalRow& z,
-                              uint32_t S, ColScalars& o) {
+                              uint32_t S, ColScalars& o, F work_free) {
   const Consts& K = C.K;
   const Derived& D = C.D;
   const spd_params_t& p = K.p;
@@ -689,6 +690,8 @@ __device__ void column_second(const ConstsD& C, float* sm, const SurfaceIn& s, c
     add_lw(1, d_last + (-corlw2));
     o.ftop_lw = (corlw1 + corlw2) + sum4(top01, fl23);
   }
+
+  work_free();
 
   // ---- get_vertical_diffusion_tend (vertical_diffusion.py:10-136) -------------------------
   // Each level's ttenvd / qtenvd is formed completely, in the reference's order, and then added

@@ -88,10 +88,10 @@ __global__ void __launch_bounds__(kNT, 5) ensemble_levelset(const __grid_constan
   }
 }
 
-template <int KX>
+template <int KX, bool kEarly, bool kVerify>
 __device__ __forceinline__ uint32_t fused_column(const ConstsD& CD, float* sm,
                                                  const MemberDev& m, const uint32_t* S, int c) {
-  return fused_process<KX>(CD, sm, m.in, m.out, S, c, m.C, m.il);
+  return fused_process<KX, kEarly, kVerify>(CD, sm, m.in, m.out, S, c, m.C, m.il);
 }
 
 // Start of a call: the level set that the last call's columns formed (T) becomes each member's
@@ -113,9 +113,18 @@ __global__ void __launch_bounds__(kNT) ensemble_begin(const __grid_constant__ Ti
 // Fused launch: every column whole (fused_process).  speculate = 1: the shortwave uses each
 // member's predicted level set P while the columns OR their own cloud tops into T; else T is
 // complete (the level-set launch formed it) and the columns read it.
-__global__ void __launch_bounds__(kNT, 4) ensemble_fused(const __grid_constant__ ClassArgs A,
-                                                         const __grid_constant__ TileSource T,
-                                                         int ntiles, int speculate) {
+// Two register budgets, which give the same bits (every operation rounds on its own): 128 for
+// four blocks per SM, what the arena of 16 levels leaves room for; or 255, with the surface fields
+// read early, where two blocks per SM hold the whole call at once (T85 with 16 levels 23.5 -> 21.7
+// us on the device, T42 with 8 levels 18.5 -> 18.1; T425 with 16 levels would take 341 against
+// 273 us).
+// kVerify: whether any class fuses verify; without it the launch carries nothing for it (T425 with 16
+// levels 268 against 277 us).
+template <int kBlocksPerSm, bool kVerify>
+__global__ void __launch_bounds__(kNT, kBlocksPerSm)
+    ensemble_fused(const __grid_constant__ ClassArgs A, const __grid_constant__ TileSource T,
+                   int ntiles, int speculate) {
+  constexpr bool kEarly = kBlocksPerSm < 4;
   extern __shared__ float sm[];
   for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
     int col0;
@@ -126,9 +135,9 @@ __global__ void __launch_bounds__(kNT, 4) ensemble_fused(const __grid_constant__
     if (c < m.C) {
       const ConstsD& CD = A.cls[m.cls];
       switch (m.kx) {
-        case 16: bit = fused_column<16>(CD, sm, m, S, c); break;
-        case 8: bit = fused_column<8>(CD, sm, m, S, c); break;
-        default: bit = fused_column<7>(CD, sm, m, S, c); break;
+        case 16: bit = fused_column<16, kEarly, kVerify>(CD, sm, m, S, c); break;
+        case 8: bit = fused_column<8, kEarly, kVerify>(CD, sm, m, S, c); break;
+        default: bit = fused_column<7, kEarly, kVerify>(CD, sm, m, S, c); break;
       }
     }
     if (speculate) or_level_set_warp(bit, m.S + LS_T * m.ls_stride);
@@ -164,13 +173,18 @@ __global__ void __launch_bounds__(kNT, 4) ensemble_fixup(const __grid_constant__
       const ConstsD& CD = A.cls[m.cls];
       const uint32_t* St = m.S + LS_T * m.ls_stride;
       switch (m.kx) {
-        case 16: fused_column<16>(CD, sm, m, St, c); break;
-        case 8: fused_column<8>(CD, sm, m, St, c); break;
-        default: fused_column<7>(CD, sm, m, St, c); break;
+        case 16: fused_column<16, false, true>(CD, sm, m, St, c); break;
+        case 8: fused_column<8, false, true>(CD, sm, m, St, c); break;
+        default: fused_column<7, false, true>(CD, sm, m, St, c); break;
       }
     }
   }
 }
+
+// The fused launch's forms: four blocks per SM without and with verify, two without and with.
+static void (*const kFused[])(const ClassArgs, const TileSource, int, int) = {
+    ensemble_fused<4, false>, ensemble_fused<4, true>, ensemble_fused<2, false>,
+    ensemble_fused<2, true>};
 
 static size_t arena_bytes(int kx) { return (size_t)kNumArrays * kx * kNT * sizeof(float); }
 
@@ -192,16 +206,18 @@ int residency(Residency& R) {
   std::lock_guard<std::mutex> lock(mu);
   if (!done[dev]) {
     Residency r;
-    if (cudaFuncSetAttribute(ensemble_fused, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem_bytes<16>()) != cudaSuccess ||
-        cudaFuncSetAttribute(ensemble_fixup, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    for (auto* kernel : kFused)
+      if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)smem_bytes<16>()) != cudaSuccess)
+        return SPD_ERR_CUDA;
+    if (cudaFuncSetAttribute(ensemble_fixup, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)smem_bytes<16>()) != cudaSuccess ||
         cudaDeviceGetAttribute(&r.sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r.lvl, ensemble_levelset, kNT, 0) !=
             cudaSuccess)
       return SPD_ERR_CUDA;
     for (int kx : {7, 8, 16})
-      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r.cols[kx], ensemble_fused, kNT,
+      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r.cols[kx], ensemble_fused<4, true>, kNT,
                                                         arena_bytes(kx)) != cudaSuccess)
         return SPD_ERR_CUDA;
     r.lvl = std::max(r.lvl, 1);
@@ -215,7 +231,8 @@ int residency(Residency& R) {
 }  // namespace
 
 int launch_forward(const ClassArgs& A, const TileSource& T, int ntiles, int kx_layout,
-                   int grid_blocks, bool speculate, cudaStream_t st, cudaEvent_t marker) {
+                   int grid_blocks, bool speculate, bool verify, cudaStream_t st,
+                   cudaEvent_t marker) {
   Residency R;
   const int rc = residency(R);
   if (rc != SPD_OK) return rc;
@@ -236,10 +253,11 @@ int launch_forward(const ClassArgs& A, const TileSource& T, int ntiles, int kx_l
   // return when no prediction missed, and a grid of one block per tile spends microseconds on
   // scheduling thousands of such blocks
   const int grid_fix = std::min(grid_cols, res_cols);
+  auto* fused = kFused[2 * (grid_cols == ntiles && ntiles <= 2 * R.sms) + verify];
   int r;
   if (speculate) {
     ensemble_begin<<<1, kNT, 0, st>>>(T);
-    r = launch_dependent(ensemble_fused, grid_cols, kNT, arena, st, A, T, ntiles, 1);
+    r = launch_dependent(fused, grid_cols, kNT, arena, st, A, T, ntiles, 1);
     if (r != SPD_OK) return r;
     if (marker) {  // timing hook: the fused launch apart, then the fixup in plain stream order
       if (cudaEventRecord(marker, st) != cudaSuccess) return SPD_ERR_CUDA;
@@ -252,10 +270,10 @@ int launch_forward(const ClassArgs& A, const TileSource& T, int ntiles, int kx_l
     ensemble_levelset<<<grid_lvl, kNT, 0, st>>>(A, T, ntiles, pf_lvl);
     if (marker) {  // timing hook: the two launches apart, in plain stream order
       if (cudaEventRecord(marker, st) != cudaSuccess) return SPD_ERR_CUDA;
-      ensemble_fused<<<grid_cols, kNT, arena, st>>>(A, T, ntiles, 0);
+      fused<<<grid_cols, kNT, arena, st>>>(A, T, ntiles, 0);
       r = SPD_OK;
     } else {
-      r = launch_dependent(ensemble_fused, grid_cols, kNT, arena, st, A, T, ntiles, 0);
+      r = launch_dependent(fused, grid_cols, kNT, arena, st, A, T, ntiles, 0);
     }
   }
   if (r != SPD_OK) return r;
@@ -265,7 +283,7 @@ int launch_forward(const ClassArgs& A, const TileSource& T, int ntiles, int kx_l
 int preload_ensemble() {
   cudaFuncAttributes a;
   bool ok = cudaFuncGetAttributes(&a, ensemble_levelset) == cudaSuccess;
-  ok &= cudaFuncGetAttributes(&a, ensemble_fused) == cudaSuccess;
+  for (auto* kernel : kFused) ok &= cudaFuncGetAttributes(&a, kernel) == cudaSuccess;
   ok &= cudaFuncGetAttributes(&a, ensemble_fixup) == cudaSuccess;
   ok &= cudaFuncGetAttributes(&a, ensemble_begin) == cudaSuccess;
   return ok ? SPD_OK : SPD_ERR_CUDA;
@@ -347,10 +365,12 @@ int spd_ensemble_fwd_marked(const spd_class_t* classes, int nclasses, void* plan
   if (kx_layout != 7 && kx_layout != 8 && kx_layout != 16) return SPD_ERR_KX;
   char* base = static_cast<char*>(plan_device);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  bool speculate = true;
-  for (int i = 0; i < nclasses; ++i)
+  bool speculate = true, verify = false;
+  for (int i = 0; i < nclasses; ++i) {
     if (classes[i].desc.flags & (SPD_ACCUMULATE_DIAGNOSTICS | SPD_NO_SPECULATION))
       speculate = false;
+    if (classes[i].desc.flags & SPD_FUSE_VERIFY) verify = true;
+  }
   const int nw = (info->nmembers + 3) & ~3;
   TileSource T{};
   T.members = reinterpret_cast<const MemberDev*>(base + 256);
@@ -358,7 +378,7 @@ int spd_ensemble_fwd_marked(const spd_class_t* classes, int nclasses, void* plan
       base + 256 + align256((size_t)info->nmembers * sizeof(MemberDev)));
   T.nmembers = info->nmembers;
   T.redone = reinterpret_cast<uint32_t*>(base + info->levelset_offset + 16 + 12 * (size_t)nw);
-  return launch_forward(A, T, info->ntiles, kx_layout, grid_blocks, speculate, st,
+  return launch_forward(A, T, info->ntiles, kx_layout, grid_blocks, speculate, verify, st,
                         static_cast<cudaEvent_t>(event));
 }
 

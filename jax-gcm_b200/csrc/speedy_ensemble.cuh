@@ -71,10 +71,12 @@ __device__ __forceinline__ void prefetch_tile_rows(int nrows, RowFn row) {
 // otherwise a level-set launch forms every T before the fused launch reads it.  grid_blocks:
 // > 0 = the fused launch's persistent grid; 0 or SPD_GRID_PER_TILE = one block per tile (the
 // 61-member ensemble takes 150 us so, 161 us as a persistent grid of SMs x resident blocks,
-// whose blocks own unequal strides of 8- and 16-level tiles).  kx_layout is the largest level count among the
+// whose blocks own unequal strides of 8- and 16-level tiles).  verify: whether any class fuses
+// verify.  kx_layout is the largest level count among the
 // tiles (it sizes the fused launch's shared-memory arena).
 int launch_forward(const ClassArgs& A, const TileSource& T, int ntiles, int kx_layout,
-                   int grid_blocks, bool speculate, cudaStream_t st, cudaEvent_t marker);
+                   int grid_blocks, bool speculate, bool verify, cudaStream_t st,
+                   cudaEvent_t marker);
 
 // Launches kernel<<<grid, threads, smem, st>>>(args...) as a programmatic dependent launch: its
 // blocks may start as the previous launch's blocks retire (they wait on the device,

@@ -103,17 +103,36 @@ __device__ __forceinline__ void orographic_horizontal(const Derived& D, float ph
   qcorh = 0.7f * (qref - qsfc);  // refrh1 (physical_constants.py:27)
 }
 
+// Starts the copies of the unclamped humidities (the levels of `neg`) to the work array, which the
+// column's radiation is done with; verify_tendencies waits for them after the vertical diffusion.
+// (Loaded there level by level, each load a wait of its own, T425 with 16 levels, verify and 2 %
+// negative humidities took 330 us, now 295.)
+template <int KX>
+__device__ __forceinline__ void fetch_clamped(float* sm, const float* q_in, uint32_t neg, int c,
+                                              int C) {
+  const uint32_t w =
+      (uint32_t)__cvta_generic_to_shared(sm + (size_t)A_W * KX * kNT + threadIdx.x);
+#pragma unroll 1
+  for (; neg; neg &= neg - 1u) {
+    const int k = __ffs(neg) - 1;
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(
+                     w + (uint32_t)(k * kNT * sizeof(float))),
+                 "l"(q_in + (size_t)k * C + c)
+                 : "memory");
+  }
+}
+
 // The end of column c, shared by the forward's kernels: the orographic correction (the last
 // term, when on), verify_tendencies, the tendency stores and the diagnostics.  The level arrays
 // T, Q (clamped by verify_state where `neg` has a bit), the accumulated tendencies DT and DQ are
 // in the block's shared-memory arena; o holds the column's scalar results.
-template <int KX>
+template <int KX, bool kVerify>
 __device__ __forceinline__ void column_outputs(const ConstsD& CD, float* sm,
                                                const spd_inputs_t& in, const spd_outputs_t& out,
                                                const SurfaceIn& s, const ColScalars& o,
                                                uint32_t neg, int c, int C) {
   const Consts& K = CD.K;
-  const bool verify = (K.flags & SPD_FUSE_VERIFY) != 0;
+  const bool verify = kVerify && (K.flags & SPD_FUSE_VERIFY) != 0;
   float* dtp = sm + (size_t)A_DT * KX * kNT + threadIdx.x;
   float* dqp = sm + (size_t)A_DQ * KX * kNT + threadIdx.x;
   if (K.flags & SPD_OROGRAPHIC) {  // the last term (get_orographic_correction_tendencies)
@@ -127,13 +146,15 @@ __device__ __forceinline__ void column_outputs(const ConstsD& CD, float* sm,
     }
   }
   const float* qp = sm + (size_t)A_Q * KX * kNT + threadIdx.x;
-  // verify_tendencies (physics_interface.py:321-342) with the unclamped humidity
+  // verify_tendencies (physics_interface.py:321-342) with the unclamped humidity, which
+  // fetch_clamped put in the work array where it was clamped
   if (verify) {
     const float dt = K.dt_seconds;
+    const float* wp = sm + (size_t)A_W * KX * kNT + threadIdx.x;
+    asm volatile("cp.async.wait_all;" ::: "memory");
 #pragma unroll 1
     for (int k = 0; k < KX; ++k) {
-      const float qr = (neg >> k & 1u) ? __ldg(in.specific_humidity + (size_t)k * C + c)
-                                       : qp[k * kNT];
+      const float qr = (neg >> k & 1u) ? wp[k * kNT] : qp[k * kNT];
       const float dq = dqp[k * kNT];
       dqp[k * kNT] = (qr + dt * dq >= 0.0f) ? dq : -qr / dt;
     }
@@ -223,13 +244,16 @@ __device__ __forceinline__ ZonalRow zonal_row_of(const Derived& D, float sia, fl
 // steady state, 25.2 us with the hint; the ensemble step went from 0.164 to 0.152 ms and the
 // T425 launch from 0.286 to 0.279 ms, results bitwise the same).
 // The level-set launch keeps the plain read-only path: the fused launch reads those rows again.
-template <int KX>
+// kEarly: the surface fields are read with the levels, before the first half, which holds them in
+// 12 registers; else after it.  kVerify: false where no column of the launch applies
+// verify_state and verify_tendencies.
+template <int KX, bool kEarly, bool kVerify>
 __device__ __forceinline__ uint32_t fused_process(const ConstsD& CD, float* sm,
                                                   const spd_inputs_t& in,
                                                   const spd_outputs_t& out, const uint32_t* S,
                                                   int c, int C, int il) {
   const Consts& K = CD.K;
-  const bool verify = (K.flags & SPD_FUSE_VERIFY) != 0;
+  const bool verify = kVerify && (K.flags & SPD_FUSE_VERIFY) != 0;
   const bool low = (K.flags & SPD_LOW_LEVEL_WINDS) != 0;
   float t[KX], q[KX], phi[KX];
   uint32_t neg = 0;
@@ -245,6 +269,24 @@ __device__ __forceinline__ uint32_t fused_process(const ConstsD& CD, float* sm,
   SurfaceIn s;
   s.psa = __ldcs(in.normalized_surface_pressure + c);
   s.fmask = __ldcs(in.fmask + c);
+  float sia, coa;
+  auto load_surface = [&] {
+    const size_t lw = low ? 0 : (size_t)(KX - 1) * C;
+    s.u_low = __ldcs(in.u_wind + lw + c);
+    s.v_low = __ldcs(in.v_wind + lw + c);
+    s.sst = __ldcs(in.sea_surface_temperature + c);
+    s.stl = __ldcs(in.stl_am + c);
+    s.soilw = __ldcs(in.soilw_am + c);
+    s.snowc = __ldcs(in.snowc_am + c);
+    s.sice = __ldcs(in.sice_am + c);
+    s.alb0 = __ldcs(in.alb0 + c);
+    s.orog = __ldcs(in.orog + c);
+    s.phis0 = __ldcs(in.phis0 + c);
+    const int j = c % il;
+    sia = __ldg(in.sia + j);
+    coa = __ldg(in.coa + j);
+  };
+  if (kEarly) load_surface();
   ColScalars o;
   {
     float qs[KX], dt[KX], dq[KX];
@@ -265,23 +307,14 @@ __device__ __forceinline__ uint32_t fused_process(const ConstsD& CD, float* sm,
       dqp[k * kNT] = dq[k];
     }
   }
-  const size_t lw = low ? 0 : (size_t)(KX - 1) * C;
-  s.u_low = __ldcs(in.u_wind + lw + c);
-  s.v_low = __ldcs(in.v_wind + lw + c);
-  s.sst = __ldcs(in.sea_surface_temperature + c);
-  s.stl = __ldcs(in.stl_am + c);
-  s.soilw = __ldcs(in.soilw_am + c);
-  s.snowc = __ldcs(in.snowc_am + c);
-  s.sice = __ldcs(in.sice_am + c);
-  s.alb0 = __ldcs(in.alb0 + c);
-  s.orog = __ldcs(in.orog + c);
-  s.phis0 = __ldcs(in.phis0 + c);
-  const int j = c % il;
-  const ZonalRow z = zonal_row_of(CD.D, __ldg(in.sia + j), __ldg(in.coa + j));
+  if (!kEarly) load_surface();
+  const ZonalRow z = zonal_row_of(CD.D, sia, coa);
   asm volatile("griddepcontrol.wait;" ::: "memory");
   const uint32_t Sw = *reinterpret_cast<const volatile uint32_t*>(S);
-  column_second<KX>(CD, sm, s, z, Sw, o);
-  column_outputs<KX>(CD, sm, in, out, s, o, neg, c, C);
+  column_second<KX>(CD, sm, s, z, Sw, o, [&] {
+    if (kVerify) fetch_clamped<KX>(sm, in.specific_humidity, neg, c, C);
+  });
+  column_outputs<KX, kVerify>(CD, sm, in, out, s, o, neg, c, C);
   return 1u << min(max(o.icltop, 0), KX - 1);
 }
 
