@@ -256,6 +256,26 @@ int spd_vjp(const spd_desc_t* desc, const spd_vgrid_t* vgrid, const spd_params_t
             void* scratch, size_t scratch_bytes, void* stream);
 
 /* ----------------------------------------------------------------------------------------- */
+/* Vector updates of an explicit column rollout x_{n+1} = x_n + dt f_n over the evolved planes   */
+/* (u, v, T, q), [kx][columns] each, and of its adjoint; one launch each.  No reference          */
+/* counterpart (the reference integrates with its dynamical core's time stepper).  Planes of one */
+/* call do not overlap, except that out may be the plane it updates (out = x, out = xbar).      */
+/* ----------------------------------------------------------------------------------------- */
+typedef struct {
+  float *u_wind, *v_wind, *temperature, *specific_humidity;
+} spd_planes_t;
+
+/* out = x + dt f (one rounding). */
+int spd_rollout_step(int32_t kx, int64_t columns, float dt, const spd_cotangents_t* x,
+                     const spd_cotangents_t* f, const spd_planes_t* out, void* stream);
+
+/* out = xbar + g and ct = dt out for the evolved planes; phi_sum += g->geopotential, psa_sum +=
+ * g->normalized_surface_pressure [columns], params_sum += g->params. */
+int spd_rollout_reverse(int32_t kx, int64_t columns, float dt, const spd_cotangents_t* xbar,
+                        const spd_grads_t* g, const spd_planes_t* out, const spd_planes_t* ct,
+                        float* phi_sum, float* psa_sum, float* params_sum, void* stream);
+
+/* ----------------------------------------------------------------------------------------- */
 /* Batched ragged ensemble: many instances ("members") of mixed resolution and level count,  */
 /* e.g. a forecast ensemble or a set of independent grids, in one fused launch over every      */
 /* member's columns (and a fixup launch that redoes the members whose predicted level set       */

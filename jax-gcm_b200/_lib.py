@@ -231,7 +231,8 @@ def calls():
                     importlib.util.spec_from_loader("_calls", loader))
                 loader.exec_module(mod)
                 mod.bind(*(C.cast(f, C.c_void_p).value
-                           for f in (lib.spd_fwd_marked, lib.spd_vjp, lib.spd_held_suarez)))
+                           for f in (lib.spd_fwd_marked, lib.spd_vjp, lib.spd_held_suarez,
+                                     lib.spd_rollout_step, lib.spd_rollout_reverse)))
                 _calls = mod
     return _calls
 

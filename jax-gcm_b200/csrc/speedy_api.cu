@@ -142,6 +142,7 @@ int dispatch_fwd(const ConstsD& CD, int kx, const spd_inputs_t& in, const spd_ou
 int preload_ensemble();
 int preload_adjoint();
 int preload_held_suarez();
+int preload_rollout();
 
 }  // namespace spd
 
@@ -151,7 +152,8 @@ int spd_preload(void) {
   const int b = spd::preload_ensemble();
   const int c = spd::preload_adjoint();
   const int h = spd::preload_held_suarez();
-  return (b == SPD_OK && c == SPD_OK && h == SPD_OK) ? SPD_OK : SPD_ERR_CUDA;
+  const int r = spd::preload_rollout();
+  return (b == SPD_OK && c == SPD_OK && h == SPD_OK && r == SPD_OK) ? SPD_OK : SPD_ERR_CUDA;
 }
 
 

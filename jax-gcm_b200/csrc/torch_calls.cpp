@@ -1,5 +1,5 @@
 // torch_calls.cpp -- the plain calls on torch tensors: gathers the field pointers, allocates the
-// results and calls the C ABI, for physics.py, adjoint.py and held_suarez.py.
+// results and calls the C ABI, for physics.py, adjoint.py, held_suarez.py and rollout.py.
 //
 // A small call is bound by the host: through ctypes a T21 call with its diagnostics took 91 us, of
 // which the device works 17 (21 torch.empty calls of 2.4 us each, 38 pointers, the structures).
@@ -14,6 +14,7 @@
 #include <torch/csrc/utils/pybind.h>
 
 #include <ATen/cuda/EmptyTensor.h>
+#include <c10/core/GradMode.h>
 #include <c10/cuda/CUDAStream.h>
 
 #include <array>
@@ -25,6 +26,8 @@ namespace {
 decltype(&spd_fwd_marked) g_fwd = nullptr;
 decltype(&spd_vjp) g_vjp = nullptr;
 decltype(&spd_held_suarez) g_hs = nullptr;
+decltype(&spd_rollout_step) g_step = nullptr;
+decltype(&spd_rollout_reverse) g_reverse = nullptr;
 
 enum Owner { kState, kForcing, kGeometry };
 struct Name {
@@ -232,13 +235,124 @@ PyObject* held_suarez(PyObject*, PyObject* const* a, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
-// bind(spd_fwd_marked, spd_vjp, spd_held_suarez): the library's entry points, as addresses.
-PyObject* bind(PyObject*, PyObject* const* a, Py_ssize_t n) {
+// The tensor attributes u_wind, v_wind, temperature and specific_humidity of an object (or the items
+// of a list) when they are what the rollout's kernels take: contiguous float32 on one CUDA device,
+// of one shape, with no gradient to record; false otherwise.
+bool planes(PyObject* obj, std::array<at::Tensor, 4>& t) {
+  for (int i = 0; i < 4; ++i) {
+    if (PyList_Check(obj)) {
+      if (PyList_GET_SIZE(obj) != 4 || !THPVariable_Check(PyList_GET_ITEM(obj, i))) return false;
+      t[i] = THPVariable_Unpack(PyList_GET_ITEM(obj, i));
+    } else {
+      t[i] = attribute(obj, g_inputs[i].str);
+    }
+    if (!t[i].is_cuda() || t[i].scalar_type() != at::kFloat || !t[i].is_contiguous() ||
+        t[i].dim() < 1 || t[i].numel() == 0 || t[i].device() != t[0].device() ||
+        t[i].sizes() != t[0].sizes() || (t[i].requires_grad() && c10::GradMode::is_enabled()))
+      return false;
+  }
+  return true;
+}
+
+template <class S>
+S pointers(const std::array<at::Tensor, 4>& t) {
+  S s;
+  auto** p = reinterpret_cast<void**>(&s);
+  for (int i = 0; i < 4; ++i) p[i] = t[i].data_ptr();
+  return s;
+}
+
+std::array<at::Tensor, 4> empty_planes(const at::Tensor& like) {
+  std::array<at::Tensor, 4> t;
+  for (at::Tensor& x : t) x = empty(like.sizes(), like.device());
+  return t;
+}
+
+// rollout_step(state, tendency, dt) -> (status, [u, v, T, q]), or None where the planes are not
+// what the kernel takes.
+PyObject* rollout_step(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   expect(n, 3);
+  std::array<at::Tensor, 4> x, f;
+  if (!planes(a[0], x) || !planes(a[1], f) || x[0].sizes() != f[0].sizes() ||
+      x[0].device() != f[0].device() || x[0].size(0) > SPD_MAX_KX)
+    Py_RETURN_NONE;
+  const double dt = PyFloat_AsDouble(a[2]);
+  if (PyErr_Occurred()) throw python_error();
+  const std::array<at::Tensor, 4> out = empty_planes(x[0]);
+  const auto px = pointers<spd_cotangents_t>(x), pf = pointers<spd_cotangents_t>(f);
+  const auto po = pointers<spd_planes_t>(out);
+  const int32_t kx = (int32_t)x[0].size(0);
+  const int64_t columns = x[0].numel() / kx;
+  void* stream = stream_of(x[0].device());
+  int rc;
+  {
+    pybind11::gil_scoped_release release;
+    rc = g_step(kx, columns, (float)dt, &px, &pf, &po, stream);
+  }
+  return result(rc, out.data(), 4);
+  END_HANDLE_TH_ERRORS
+}
+
+// rollout_reverse(xbar, gradients, params, phi_sum, psa_sum, params_sum, dt)
+//   -> (status, [four xbar planes, four cotangent planes]), or None where they are not what the
+// kernel takes.  xbar: four planes; gradients: a PhysicsState; the sums are added to in place.
+PyObject* rollout_reverse(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  expect(n, 7);
+  std::array<at::Tensor, 4> xb, g;
+  if (!planes(a[0], xb) || !planes(a[1], g) || xb[0].sizes() != g[0].sizes() ||
+      xb[0].device() != g[0].device() || xb[0].size(0) > SPD_MAX_KX)
+    Py_RETURN_NONE;
+  const at::Tensor g_phi = attribute(a[1], g_inputs[4].str), g_psa = attribute(a[1], g_inputs[5].str);
+  std::array<at::Tensor, 6> rest = {g_phi, g_psa};
+  for (int i = 0; i < 4; ++i) {
+    TORCH_CHECK_TYPE(THPVariable_Check(a[2 + i]), "expected a tensor");
+    rest[2 + i] = THPVariable_Unpack(a[2 + i]);
+  }
+  const int32_t kx = (int32_t)xb[0].size(0);
+  const int64_t columns = xb[0].numel() / kx;
+  const int64_t want[] = {kx * columns, columns, SPD_NUM_DIFF_PARAMS, kx * columns, columns,
+                          SPD_NUM_DIFF_PARAMS};
+  for (int i = 0; i < 6; ++i)
+    if (rest[i].device() != xb[0].device() || rest[i].scalar_type() != at::kFloat ||
+        !rest[i].is_contiguous() || rest[i].numel() != want[i])
+      Py_RETURN_NONE;
+  const double dt = PyFloat_AsDouble(a[6]);
+  if (PyErr_Occurred()) throw python_error();
+  std::array<at::Tensor, 8> t;
+  const std::array<at::Tensor, 4> out = empty_planes(xb[0]), ct = empty_planes(xb[0]);
+  for (int i = 0; i < 4; ++i) {
+    t[i] = out[i];
+    t[4 + i] = ct[i];
+  }
+  const auto px = pointers<spd_cotangents_t>(xb);
+  const auto po = pointers<spd_planes_t>(out), pc = pointers<spd_planes_t>(ct);
+  auto w = [&](int i) { return static_cast<float*>(rest[i].data_ptr()); };
+  const spd_grads_t pg = {static_cast<float*>(g[0].data_ptr()), static_cast<float*>(g[1].data_ptr()),
+                          static_cast<float*>(g[2].data_ptr()), static_cast<float*>(g[3].data_ptr()),
+                          w(0), w(1), w(2)};
+  float *phi = w(3), *psa = w(4), *par = w(5);
+  void* stream = stream_of(xb[0].device());
+  int rc;
+  {
+    pybind11::gil_scoped_release release;
+    rc = g_reverse(kx, columns, (float)dt, &px, &pg, &po, &pc, phi, psa, par, stream);
+  }
+  return result(rc, t.data(), 8);
+  END_HANDLE_TH_ERRORS
+}
+
+// bind(spd_fwd_marked, spd_vjp, spd_held_suarez, spd_rollout_step, spd_rollout_reverse): the
+// library's entry points, as addresses.
+PyObject* bind(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  expect(n, 5);
   g_fwd = reinterpret_cast<decltype(g_fwd)>(address<void>(a[0]));
   g_vjp = reinterpret_cast<decltype(g_vjp)>(address<void>(a[1]));
   g_hs = reinterpret_cast<decltype(g_hs)>(address<void>(a[2]));
+  g_step = reinterpret_cast<decltype(g_step)>(address<void>(a[3]));
+  g_reverse = reinterpret_cast<decltype(g_reverse)>(address<void>(a[4]));
   Py_RETURN_NONE;
   END_HANDLE_TH_ERRORS
 }
@@ -250,7 +364,9 @@ PyMethodDef method(const char* name) {
 }
 
 PyMethodDef g_methods[] = {method<fwd>("fwd"), method<vjp>("vjp"),
-                           method<held_suarez>("held_suarez"), method<bind>("bind"),
+                           method<held_suarez>("held_suarez"),
+                           method<rollout_step>("rollout_step"),
+                           method<rollout_reverse>("rollout_reverse"), method<bind>("bind"),
                            {nullptr, nullptr, 0, nullptr}};
 PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "_calls", nullptr, -1, g_methods,
                         nullptr, nullptr, nullptr, nullptr};

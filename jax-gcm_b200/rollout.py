@@ -27,6 +27,7 @@ from typing import Optional
 
 import torch
 
+from . import _lib
 from .adjoint import vjp
 from .physics import PhysicsState, PhysicsTendency, SpeedyPhysics
 
@@ -46,11 +47,16 @@ def _date(date, n):
 
 def step(physics: SpeedyPhysics, state: PhysicsState, forcing, geometry, date, dt: float):
     """One explicit step of the fused physics: a new PhysicsState (the four Euler updates in
-    one multi-tensor launch)."""
+    one launch)."""
     tend, _ = physics.compute_tendencies(state, forcing, geometry, date)
-    u, v, t, q = torch._foreach_add([getattr(state, k) for k in EVOLVED],
+    done = _lib.calls().rollout_step(state, tend, dt) if state.temperature.is_cuda else None
+    if done is None:  # other dtypes, strides or devices, or a gradient to record
+        planes = torch._foreach_add([getattr(state, k) for k in EVOLVED],
                                     [getattr(tend, k) for k in EVOLVED], alpha=dt)
-    return PhysicsState(u, v, t, q, state.geopotential, state.normalized_surface_pressure)
+    else:
+        _lib.check(done[0], "spd_rollout_step")
+        planes = done[1]
+    return PhysicsState(*planes, state.geopotential, state.normalized_surface_pressure)
 
 
 def rollout(physics, state, forcing, geometry, date, nsteps=48, dt=1800.0):
@@ -119,17 +125,22 @@ def rollout_vjp(physics, state, forcing, geometry, date, cotangent, nsteps=48, d
     def fwd(x, n):
         return step(ph, x, forcing, geometry, _date(date, n), dt)
 
-    def rev(x, n, xb):
-        ct = PhysicsTendency(*torch._foreach_mul([xb[k] for k in EVOLVED], dt))
-        g, gp = vjp(ph, x, forcing, geometry, _date(date, n), ct)
-        # the fixed fields' and the parameters' gradients accumulate in place, in one launch
-        torch._foreach_add_([phi_b, psa_b, par_b], [g.geopotential, g.normalized_surface_pressure,
-                                                   gp])
-        return dict(zip(EVOLVED, torch._foreach_add([xb[k] for k in EVOLVED],
-                                                    [getattr(g, k) for k in EVOLVED])))
+    def rev(x, n, bar):
+        xb, ct = bar  # the state's adjoint, and dt times it: the step's cotangent
+        g, gp = vjp(ph, x, forcing, geometry, _date(date, n), PhysicsTendency(*ct))
+        # the state's adjoint, the next cotangent, and the sums of the fixed fields' and the
+        # parameters' gradients (in place), in one launch
+        done = calls.rollout_reverse(xb, g, gp, phi_b, psa_b, par_b, dt)
+        if done is None:
+            torch._foreach_add_([phi_b, psa_b, par_b],
+                                [g.geopotential, g.normalized_surface_pressure, gp])
+            xb = list(torch._foreach_add(xb, [getattr(g, k) for k in EVOLVED]))
+            return xb, torch._foreach_mul(xb, dt)
+        _lib.check(done[0], "spd_rollout_reverse")
+        return done[1][:4], done[1][4:]
 
-    xb0 = {k: getattr(cotangent, k).to(torch.float32).clone() for k in EVOLVED}
-    final, xb, _ = checkpointed_reverse(fwd, rev, state, xb0, nsteps, checkpoint_every)
-    grads = PhysicsState(xb["u_wind"], xb["v_wind"], xb["temperature"], xb["specific_humidity"],
-                         phi_b, psa_b)
-    return final, grads, par_b
+    calls = _lib.calls()
+    xb0 = [getattr(cotangent, k).to(torch.float32).clone() for k in EVOLVED]
+    final, (xb, _), _ = checkpointed_reverse(fwd, rev, state, (xb0, torch._foreach_mul(xb0, dt)),
+                                             nsteps, checkpoint_every)
+    return final, PhysicsState(*xb, phi_b, psa_b), par_b
