@@ -112,7 +112,10 @@ __global__ void __launch_bounds__(kBlock)
 //    96 registers with twenty warps 442 us at T425 but 110 against 96 us at T170);
 //  - 255 (eight), which spills next to nothing, where two warps per scheduler hold the whole batch
 //    (T85 with 16 levels, 1,024 warps: 60 against 66 us; T170, 4,096 warps: 209 against 194 us).
-template <int kWarpsPerSm>
+// kVerify: whether any class fuses verify; without it the launch carries neither the limited levels
+// nor the humidity tendencies they are found from (T425 with 16 levels 887 against 934
+// us, T85 49.5 against 53.2).
+template <int kWarpsPerSm, bool kVerify>
 __global__ void __launch_bounds__(kNT, kWarpsPerSm / (kNT / 32))
     ensemble_adjoint(const __grid_constant__ ClassArgs A, const __grid_constant__ VjpSource T,
                      int ntiles) {
@@ -137,15 +140,21 @@ __global__ void __launch_bounds__(kNT, kWarpsPerSm / (kNT / 32))
     for (int j = 0; j < SPD_NUM_DIFF_PARAMS; ++j) pacc[j] = 0.0f;
     const ConstsD& CD = A.cls[m.cls];
     switch (m.kx) {  // uniform per block
-      case 16: column_vjp_smem<16>(CD, sm, m, c, C, valid, pacc); break;
-      case 8: column_vjp_smem<8>(CD, sm, m, c, C, valid, pacc); break;
-      default: column_vjp_smem<7>(CD, sm, m, c, C, valid, pacc); break;
+      case 16: column_vjp_smem<16, kVerify>(CD, sm, m, c, C, valid, pacc); break;
+      case 8: column_vjp_smem<8, kVerify>(CD, sm, m, c, C, valid, pacc); break;
+      default: column_vjp_smem<7, kVerify>(CD, sm, m, c, C, valid, pacc); break;
     }
 #pragma unroll
     for (int j = 0; j < SPD_NUM_DIFF_PARAMS; ++j) pacc[j] = valid ? pacc[j] : 0.0f;
     warp_add_params(pacc, load_field(m.gr.params));
   }
 }
+
+// The adjoint launch's forms: by warps per SM, without and with verify.
+enum { kWarps8, kWarps12, kWarps16 };
+static void (*const kAdjoint[])(const ClassArgs, const VjpSource, int) = {
+    ensemble_adjoint<8, false>,  ensemble_adjoint<8, true>,  ensemble_adjoint<12, false>,
+    ensemble_adjoint<12, true>, ensemble_adjoint<16, false>, ensemble_adjoint<16, true>};
 
 // Allows the adjoint launch its arena on the current device, once per device (the attribute is a
 // per-device setting of the kernel); gives the device's SM count.
@@ -159,7 +168,7 @@ static int allow_arena(int* sms = nullptr) {
   if (!count[dev]) {
     const int bytes = (int)vjp_arena_bytes(SPD_MAX_KX);
     int n = 0;
-    for (auto* kernel : {ensemble_adjoint<8>, ensemble_adjoint<12>, ensemble_adjoint<16>})
+    for (auto* kernel : kAdjoint)
       if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) !=
           cudaSuccess)
         return SPD_ERR_CUDA;
@@ -185,14 +194,15 @@ int preload_adjoint() {
   bool ok = true;
   ok &= cudaFuncGetAttributes(&a, vjp_begin) == cudaSuccess;
   ok &= cudaFuncGetAttributes(&a, ensemble_vjp_prepass) == cudaSuccess;
-  for (auto* kernel : {ensemble_adjoint<8>, ensemble_adjoint<12>, ensemble_adjoint<16>})
+  for (auto* kernel : kAdjoint)
     ok &= cudaFuncGetAttributes(&a, kernel) == cudaSuccess;
   return ok && allow_arena() == SPD_OK ? SPD_OK : SPD_ERR_CUDA;
 }
 
 // The three launches; each but the first may start while the one before it runs.
-static int launch_ensemble_vjp(const ClassArgs& A, int kx_layout, const VjpSource& T, int ntiles,
-                               int grid_blocks, cudaStream_t st) {
+static int launch_ensemble_vjp(const ClassArgs& A, int kx_layout, bool verify,
+                               const VjpSource& T, int ntiles, int grid_blocks,
+                               cudaStream_t st) {
   // Default: one block per tile.  The blocks are short (one tile's columns each), so the SMs
   // turn over often and a higher-priority stream's kernels (a forward batch) get them within
   // one block's time; a persistent grid would hold every SM until the whole batch is done.
@@ -203,10 +213,8 @@ static int launch_ensemble_vjp(const ClassArgs& A, int kx_layout, const VjpSourc
   vjp_begin<<<1, kBlock, 0, st>>>(T);
   int rc = launch_dependent(ensemble_vjp_prepass, grid_pre, kBlock, 0, st, A, T, ntiles);
   if (rc != SPD_OK) return rc;
-  auto* kernel = grid * (kNT / 32) <= 8 * sms ? ensemble_adjoint<8>
-                 : kx_layout > 8              ? ensemble_adjoint<12>
-                                              : ensemble_adjoint<16>;
-  rc = launch_dependent(kernel, grid, kNT, vjp_arena_bytes(kx_layout), st, A, T, ntiles);
+  const int warps = grid * (kNT / 32) <= 8 * sms ? kWarps8 : kx_layout > 8 ? kWarps12 : kWarps16;
+  rc = launch_dependent(kAdjoint[2 * warps + verify], grid, kNT, vjp_arena_bytes(kx_layout), st, A, T, ntiles);
   if (rc != SPD_OK) return rc;
   return cudaGetLastError() == cudaSuccess ? SPD_OK : SPD_ERR_CUDA;
 }
@@ -265,7 +273,7 @@ int spd_vjp(const spd_desc_t* desc, const spd_vgrid_t* vgrid, const spd_params_t
   T.single.S = reinterpret_cast<uint32_t*>(base + L.levelset);
   T.single.table = reinterpret_cast<ZonalRow*>(base + L.tables);
   T.nmembers = 1;
-  return launch_ensemble_vjp(A, desc->kx, T, L.ntiles, 0, st);
+  return launch_ensemble_vjp(A, desc->kx, (desc->flags & SPD_FUSE_VERIFY) != 0, T, L.ntiles, 0, st);
 }
 
 size_t spd_ensemble_vjp_plan_bytes(const spd_vjp_member_t* members, int nmembers) {
@@ -321,7 +329,9 @@ int spd_ensemble_vjp(const spd_class_t* classes, int nclasses, void* plan_device
   if (nclasses <= 0 || nclasses > SPD_MAX_CLASSES || info->ntiles <= 0) return SPD_ERR_SHAPE;
   ClassArgs A;
   int kx_layout = 0;
+  bool verify = false;
   for (int i = 0; i < nclasses; ++i) {
+    if (classes[i].desc.flags & SPD_FUSE_VERIFY) verify = true;
     A.cls[i].K = make_consts(&classes[i].desc, &classes[i].vgrid, &classes[i].params);
     A.cls[i].D = derive_constants(&classes[i].desc, &classes[i].vgrid, &classes[i].params);
     kx_layout = std::max(kx_layout, classes[i].desc.kx);
@@ -332,7 +342,7 @@ int spd_ensemble_vjp(const spd_class_t* classes, int nclasses, void* plan_device
   T.tiles = reinterpret_cast<const Tile*>(
       base + 256 + align256((size_t)info->nmembers * sizeof(VjpMemberDev)));
   T.nmembers = info->nmembers;
-  return launch_ensemble_vjp(A, kx_layout, T, info->ntiles, grid_blocks,
+  return launch_ensemble_vjp(A, kx_layout, verify, T, info->ntiles, grid_blocks,
                              static_cast<cudaStream_t>(stream));
 }
 
