@@ -30,16 +30,15 @@ sys.path.insert(0, ROOT)
 
 # DRAM bytes (read + write) per column of the dominant kernel (ensemble_fused) and its warp
 # instructions per launch, from one ncu capture each (the summaries under profiles/ give the
-# commands): T425 from a --set full capture of one plain call (196.8 MB read + 174.2 MB
-# written, 216.9 M warp instructions); the ensemble from the dram__bytes / inst_executed
-# metrics of one fused launch of the benchmark's step (96.2 MB read + 60.4 MB written, 103.8 M
-# warp instructions; one block per tile, the autotuner's pick); the adjoint (ensemble_adjoint, T170
-# with 16 levels) from a --set full capture of one VJP.  Part of each launch's writes is still
+# commands): T425, one plain call (196.7 MB read + 168.6 MB written, 212.7 M warp instructions);
+# the ensemble, one fused launch of the benchmark's step (96.2 MB read + 54.7 MB written, 101.7 M
+# warp instructions; one block per tile); the adjoint (ensemble_adjoint, T170 with 16 levels), one
+# VJP.  Part of each launch's writes is still
 # in L2 when the kernel ends, so the write share reads low.
-NCU_TRAFFIC_PER_COLUMN = {"ensemble": (96.215296e6 + 60.369920e6) / 466944,
-                          "t425": (196.767232e6 + 174.180096e6) / 819200}
-NCU_WARP_INSTRUCTIONS = {"ensemble": 103782785.0, "t425": 216850069.0,
-                         "adjoint_t170": 129642118.0}
+NCU_TRAFFIC_PER_COLUMN = {"ensemble": (96.185856e6 + 54.689792e6) / 466944,
+                          "t425": (196.726784e6 + 168.578816e6) / 819200}
+NCU_WARP_INSTRUCTIONS = {"ensemble": 101748554.0, "t425": 212669550.0,
+                         "adjoint_t170": 76210642.0}
 
 
 def parse_args():
@@ -231,12 +230,12 @@ def run_b200(args):
         def step(marker=None):
             ens.forward(marker=marker)
 
-        launches_per_step = 2
+        launches_per_step = 3  # level-set roll-over, fused, fixup
     else:
         def step(marker=None):
             step_plain()
 
-        launches_per_step = 2 * len(runs)
+        launches_per_step = 3 * len(runs)
 
     def barrier():
         if dist is not None:
@@ -315,7 +314,7 @@ def run_b200(args):
     if args.mode == "batched" and not args.no_plain:
         pms = timed(step_plain, args.steps, args.warmup) / args.steps
         plain = {"value": round(cols * world / (pms / 1e3), 1), "ms_per_step": round(pms, 4),
-                 "launches_per_step": 2 * len(runs),
+                 "launches_per_step": 3 * len(runs),
                  "batched_over_plain": round(pms / ms_step, 2)}
 
     # Roofline of the dominant kernel, ensemble_fused (every column whole): the path's

@@ -165,12 +165,12 @@ int spd_fwd(const spd_desc_t* desc, const spd_vgrid_t* vgrid, const spd_params_t
             size_t scratch_bytes, void* stream);
 
 /* Timing hook (no reference counterpart): spd_fwd, recording `event` (a cudaEvent_t, or NULL)
- * on `stream` between its two launches, so that a caller can time them separately with
- * events: after the fused launch (before the fixup) when the call predicts the level set,
- * after the level-set launch (before the fused one) under SPD_NO_SPECULATION.  With an event
- * the launches run in plain stream order; without one (and in spd_fwd) the second launch is a
- * programmatic dependent launch: its blocks start as the first one's retire and wait on the
- * device for the first launch's completion before reading what it wrote. */
+ * on `stream` between the fused launch and the one beside it, so that a caller can time them
+ * separately with events: after the fused launch (before the fixup) when the call predicts the
+ * level set, after the level-set launch (before the fused one) under SPD_NO_SPECULATION.  With an
+ * event the launch after it runs in plain stream order; without one (and in spd_fwd) it is a
+ * programmatic dependent launch: its blocks start as the ones before it retire and wait on the
+ * device for that launch's completion before reading what it wrote. */
 int spd_fwd_marked(const spd_desc_t* desc, const spd_vgrid_t* vgrid, const spd_params_t* params,
                    const spd_inputs_t* in, const spd_outputs_t* out, void* scratch,
                    size_t scratch_bytes, void* stream, void* event);
@@ -227,10 +227,10 @@ int spd_held_suarez(const spd_hs_desc_t* desc, const float* lat_tab, const float
 /* derivative 0.5/0.5 (JAX's lax.min/lax.max rule); integer levels and the instance level set */
 /* carry no derivative.  With SPD_FUSE_VERIFY set the VJP is that of the fused step           */
 /* (verify_state, the physics, verify_tendencies and the humidity scale), and the humidity   */
-/* gradient is with respect to the humidity as given.  `scratch` holds a one-member plan (the  */
-/* instance's tile list, level-set word and per-latitude solar table), so that a single       */
-/* instance runs the batched adjoint's kernels: spd_vjp_scratch_bytes(desc) bytes, 256-byte   */
-/* aligned.                                                                                   */
+/* gradient is with respect to the humidity as given.  A gradient plane may be the same buffer */
+/* as an input or cotangent plane.  `scratch` is laid out like a one-member plan of the batched */
+/* adjoint, whose kernels a single instance runs; the call uses its level-set word and its     */
+/* per-latitude solar table: spd_vjp_scratch_bytes(desc) bytes, 256-byte aligned.              */
 /* ----------------------------------------------------------------------------------------- */
 #define SPD_NUM_DIFF_PARAMS 12
 
@@ -329,7 +329,7 @@ int spd_ensemble_fwd(const spd_class_t* classes, int nclasses, void* plan_device
                      const spd_plan_info_t* info, int grid_blocks, void* stream);
 
 /* Timing hook (no reference counterpart): spd_ensemble_fwd, recording `event` (a cudaEvent_t,
- * or NULL) on `stream` between its two launches (see spd_fwd_marked), which then run in plain
+ * or NULL) on `stream` beside its fused launch (see spd_fwd_marked); the launch after it is in plain
  * stream order. */
 int spd_ensemble_fwd_marked(const spd_class_t* classes, int nclasses, void* plan_device,
                             const spd_plan_info_t* info, int grid_blocks, void* stream,

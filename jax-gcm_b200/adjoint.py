@@ -4,7 +4,7 @@
 (jcm/physics/speedy/speedy_physics.py:88-127) for the tendency outputs: given cotangents of the
 four tendency planes it returns the gradients with respect to the PhysicsState planes and to
 the 12 tuning parameters (params.py:11-16, :51-54, :72-73).  It runs ``spd_vjp``, which
-recomputes each column's forward on a per-thread tape instead of storing the forward.
+recomputes each column's forward instead of storing it.
 
 ``speedy_b200::tendencies`` is the same forward as a ``torch.library`` custom op whose autograd
 rule is ``spd_vjp``; ``SpeedyTendencies`` wraps it for PhysicsState inputs.

@@ -19,7 +19,7 @@
 // vertical diffusion) needs the instance's level set of cloud tops and resumes from what the
 // first half left (qsat, the tendency accumulators, a few scalars).  The forward runs both in
 // one launch (speedy_kernels.cuh, fused_process), with the level set predicted from the
-// previous call and checked by the launch's last block (a fixup launch redoes a missed
+// previous call and checked by the launch that follows (the fixup, which redoes a missed
 // instance), or, under SPD_NO_SPECULATION, after a light launch that forms the level set from
 // column_first<KX, true>.
 //

@@ -1,5 +1,5 @@
 // speedy_ensemble.cu -- the batched ragged ensemble: many members of mixed resolution and
-// level count in two persistent launches over one tile list.
+// level count in one fused launch over one tile list (and what starts and checks it).
 //
 // A member is one grid instance (its own arrays, ix*il columns, kx levels).  The plan splits
 // every member into tiles of kNT consecutive columns (a tile never straddles members), ordered
@@ -17,7 +17,7 @@
 //   level set first (accumulating calls, which must not add a column's diagnostics twice, and
 //     calls that ask for no prediction): a light launch forms every member's S from the
 //     cloud-top part of every column, then the fused launch reads it.
-// The launches are persistent or one block per tile (gridDim blocks stride over the tile
+// The launches take one block per tile or are persistent (gridDim blocks stride over the tile
 // list).  The plain per-instance forward (spd_fwd) runs the same kernels over a one-member
 // plan given by value, so that the two paths agree bitwise.
 // Constants shared by a class of members (kx, date, switches, vertical grid, parameters) travel
