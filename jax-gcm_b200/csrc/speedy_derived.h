@@ -17,6 +17,7 @@ struct Derived {
   float rsig[SPD_MAX_KX];     // 1/dhs                                (vertical_diffusion.py:54)
   float rsig1[SPD_MAX_KX];    // 1/(1-hsg[k+1]), 0 at kx-1            (vertical_diffusion.py:55-56)
   float entr[SPD_MAX_KX];     // scaled entrainment, k = 1..kx-2      (convection.py:135-137)
+  float entu[SPD_MAX_KX];     // its derivative with respect to entmax
   float rhref[SPD_MAX_KX];    // LSC RH threshold                     (large_scale_condensation.py:298-299)
   float dqmax[SPD_MAX_KX];    // LSC max tendency                     (large_scale_condensation.py:300)
   float pfact[SPD_MAX_KX];    // dhs * p0/g                           (large_scale_condensation.py:314)
@@ -60,7 +61,10 @@ inline Derived derive_constants(const spd_desc_t* d, const spd_vgrid_t* vg,
     sentr = sentr + D.entr[k];
   }
   const float escale = p->entmax / sentr;
-  for (int k = 1; k < kx - 1; ++k) D.entr[k] = D.entr[k] * escale;
+  for (int k = 1; k < kx - 1; ++k) {
+    D.entu[k] = D.entr[k] / sentr;
+    D.entr[k] = D.entr[k] * escale;
+  }
   D.fm0 = 1e5f * vg->dhs[kx - 1] / (9.81f * p->trcnv * 3600.0f);
   D.rdps = 2.0f / (1.0f - p->psmin);
   D.rtlsc = 1.0f / (p->trlsc * 3600.0f);

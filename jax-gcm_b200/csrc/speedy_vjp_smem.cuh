@@ -1258,7 +1258,7 @@ __device__ __forceinline__ void column_vjp_smem(const ConstsD& CD, float* sm,
           se_b = CSB * en;
           qk_b = CQB * en;
           cbmf_b = fmaf(en_b, ep, cbmf_b);
-          ent_b = fmaf(en_b, D.entr[k], ent_b);
+          ent_b = fmaf(en_b, D.entu[k], ent_b);
           const float qs_k = QS[k];
           const float d0 = p.rhil * qs_k - q_k;
           if (d0 > 0.0f) {
@@ -1351,8 +1351,9 @@ __device__ __forceinline__ void column_vjp_smem(const ConstsD& CD, float* sm,
       TB[B] = fmaf(kCp, seb_m, TB[B]);
       PB[B] = PB[B] + seb_m;
       QB[B] = QB[B] + qbb_m;
-      psa_b = fmaf(ent_b, cbmf, psa_b);
-      par[spdvjp::P_ENTMAX] += fdiv(ent_b * cbmf * psa, p.entmax);
+      // the entrainment is entmax * entu: entmax may be zero
+      psa_b = fmaf(ent_b * p.entmax, cbmf, psa_b);
+      par[spdvjp::P_ENTMAX] += ent_b * cbmf * psa;
     }
   }
 
