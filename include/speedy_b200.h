@@ -191,6 +191,12 @@ int spd_preload(void);
  * on the current device's default stream. */
 int spd_selftest_packed(int n, uint32_t seed, unsigned int* mismatches);
 
+/* The adjoint's division on the caller's operands (no reference counterpart): out receives n
+ * floats each of a[i] / b[i] and 1 / b[i] by the steps that the reverse pass uses in place of
+ * IEEE division, and of a[i] / b[i] by the form that it uses where the divisor may be zero or
+ * infinite, compiled with its flags.  a, b and out (3 n floats) are on the device. */
+int spd_selftest_division(int n, const float* a, const float* b, float* out, void* stream);
+
 /* ----------------------------------------------------------------------------------------- */
 /* Held-Suarez forcing: HeldSuarezPhysics.compute_tendencies                                 */
 /*   (jcm/physics/held_suarez/held_suarez_physics.py:76-101), the reference's second physics */

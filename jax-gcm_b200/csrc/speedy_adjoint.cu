@@ -24,6 +24,7 @@
 
 // the column's first half divides like the rest of the adjoint (speedy_vjp.h, fdiv)
 #define SPD_DIV(a, b) (spdvjp::fdiv((a), (b)))
+#define SPD_DIV_FULL(a, b) (spdvjp::fdiv_full((a), (b)))
 #include "speedy_ensemble.cuh"
 #include "speedy_vjp_smem.cuh"
 
@@ -178,6 +179,17 @@ static int allow_arena(int* sms = nullptr) {
   }
   if (sms) *sms = count[dev];
   return SPD_OK;
+}
+
+// The column's divisions and reciprocal as this file compiles them (spd_selftest_division).
+__global__ void __launch_bounds__(kBlock)
+    selftest_division(int n, const float* a, const float* b, float* out) {
+  const int i = blockIdx.x * kBlock + threadIdx.x;
+  if (i >= n) return;
+  const size_t m = n;
+  out[i] = spdvjp::fdiv(a[i], b[i]);
+  out[m + i] = spdvjp::frcp(b[i]);
+  out[2 * m + i] = spdvjp::fdiv_full(a[i], b[i]);
 }
 
 struct OneMember {
@@ -344,6 +356,15 @@ int spd_ensemble_vjp(const spd_class_t* classes, int nclasses, void* plan_device
   T.nmembers = info->nmembers;
   return launch_ensemble_vjp(A, kx_layout, verify, T, info->ntiles, grid_blocks,
                              static_cast<cudaStream_t>(stream));
+}
+
+int spd_selftest_division(int n, const float* a, const float* b, float* out, void* stream) {
+  using namespace spd;
+  if (!a || !b || !out) return SPD_ERR_NULL;
+  if (n <= 0 || n > (1 << 28)) return SPD_ERR_SHAPE;
+  selftest_division<<<(n + kBlock - 1) / kBlock, kBlock, 0, static_cast<cudaStream_t>(stream)>>>(
+      n, a, b, out);
+  return cudaGetLastError() == cudaSuccess ? SPD_OK : SPD_ERR_CUDA;
 }
 
 }  // extern "C"

@@ -16,6 +16,7 @@
 // it names another (speedy_adjoint.cu).
 #ifndef SPD_DIV
 #define SPD_DIV(a, b) ((a) / (b))
+#define SPD_DIV_FULL(a, b) ((a) / (b))  // where the divisor may be zero
 #endif
 
 namespace spd {

@@ -388,7 +388,7 @@ __device__ __forceinline__ void column_first(const ConstsD& C, const float (&T)[
       o.icltop = min(iptop, icl);
       return;
     }
-    const float gse = SPD_DIV(se_b1 - se_b, PHI[KX - 2] - PHI[KX - 1]);
+    const float gse = SPD_DIV_FULL(se_b1 - se_b, PHI[KX - 2] - PHI[KX - 1]);
     const float pr1 = fminf(p.pmaxcl, 86.4f * (o.precnv + o.precls));
     cloudc = fminf(1.0f, p.wpcl * sqrtf(fmaxf(kEpsilon, pr1)) + sq(fminf(1.0f, cmax * D.rrcl)));
     if (isnan(cloudc)) cloudc = 1.0f;

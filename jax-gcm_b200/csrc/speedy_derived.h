@@ -27,6 +27,7 @@ struct Derived {
   uint32_t vdcond;            // bit k: hsg[k+1] > 0.5                (vertical_diffusion.py:100)
   float fm0, rdps;            // convection.py:140-141
   float rtlsc;                // large_scale_condensation.py:285
+  float fm0_t, rtlsc_t;       // minus their derivatives with respect to trcnv and trlsc
   float fshcq, fshcse, fvdise, drh0, fvdiq2;  // vertical_diffusion.py:45-60
   float eps1;                 // shortwave_radiation.py:203
   float rhdrag;               // surface_flux.py:311
@@ -68,6 +69,8 @@ inline Derived derive_constants(const spd_desc_t* d, const spd_vgrid_t* vg,
   D.fm0 = 1e5f * vg->dhs[kx - 1] / (9.81f * p->trcnv * 3600.0f);
   D.rdps = 2.0f / (1.0f - p->psmin);
   D.rtlsc = 1.0f / (p->trlsc * 3600.0f);
+  D.fm0_t = D.fm0 / p->trcnv;
+  D.rtlsc_t = D.rtlsc / p->trlsc;
   const float prg = (float)(1e5 / 9.81);
   for (int k = 0; k < kx; ++k) {
     const float sig2 = vg->fsg[k] * vg->fsg[k];

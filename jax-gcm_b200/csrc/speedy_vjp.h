@@ -45,19 +45,34 @@ SPD_HD bool fnan(double x) { return x != x; }
 // quotient corrected by its own residual (Markstein), which rounds like the IEEE quotient for
 // operands far from the ends of the exponent range, without the subroutine call of the IEEE one
 // (around which the compiler saves and restores registers).
+// fdiv and frcp are for operands that the column's physics keeps finite and away from zero: where
+// the steps meet 0 * inf (a zero or infinite operand, a quotient that overflows) they give NaN.
+// fdiv_full keeps the estimate's own result there, which is the IEEE one: for a divisor that may be
+// zero or infinite.  It waits for one more comparison (in fdiv's place everywhere: T425 with 16
+// levels 941 against 889 us, T85 55.1 against 51.2).
+// Neither is IEEE where the divisor is below 2^-126 (it counts as zero) or above 2^126 (as infinite),
+// and a quotient or residual that is subnormal may be off by an ulp.
 #if defined(__CUDA_ARCH__)
-SPD_HD float frcp(float b) {
+SPD_HD float rcp_estimate(float b) {
   float r;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(b));
-  return fmaf(fmaf(-b, r, 1.0f), r, r);
+  return r;
 }
-SPD_HD float fdiv(float a, float b) {
-  const float r = frcp(b), q = a * r;
+SPD_HD float rcp_refined(float b, float e) { return fmaf(fmaf(-b, e, 1.0f), e, e); }
+SPD_HD float div_refined(float a, float b, float r) {
+  const float q = a * r;
   return fmaf(fmaf(-b, q, a), r, q);
+}
+SPD_HD float frcp(float b) { return rcp_refined(b, rcp_estimate(b)); }
+SPD_HD float fdiv(float a, float b) { return div_refined(a, b, frcp(b)); }
+SPD_HD float fdiv_full(float a, float b) {
+  const float e = rcp_estimate(b), v = div_refined(a, b, rcp_refined(b, e));
+  return fnan(v) ? a * e : v;
 }
 #else
 SPD_HD float frcp(float b) { return 1.0f / b; }
 SPD_HD float fdiv(float a, float b) { return a / b; }
+SPD_HD float fdiv_full(float a, float b) { return a / b; }
 #endif
 SPD_HD double fdiv(double a, double b) { return a / b; }
 
@@ -1216,6 +1231,7 @@ struct Sf {
   F dths_v, denv2, qs11, qs11_t, qs11_p, q1_1, cdsdv, qss, qss_t, qss_p;
   F ustr0, vstr0, shf0, evap0, rlus0, ustr1, vstr1, shf1, evap1;
   F ustr2, vstr2, shf2, evap2, rps;
+  F rdth, rhdrag;  // fstab / dtheta and 1 / (9.81 hdrag): set by the caller of surface()
 };
 
 struct SurfaceIn {
@@ -1233,7 +1249,6 @@ SPD_HD void surface(const Ctx& x, Col<KX, F>& c, const SurfaceIn& s, const Surfa
   w.u0 = F(p.fwind0) * c.u;
   w.v0 = F(p.fwind0) * c.v;
   const F astab = (x.flags & SPD_LSCASYM) ? F(0.5) : F(1.0);
-  const F rdth = fdiv(F(p.fstab), F(p.dtheta));
   const bool land = (x.flags & SPD_LFLUXLAND) != 0;
   w.ustr0 = w.ustr1 = w.vstr0 = w.vstr1 = w.shf0 = w.evap0 = w.rlus0 = F(0);
   w.t1_1 = w.q1_1 = w.denv2 = F(0);
@@ -1265,10 +1280,9 @@ SPD_HD void surface(const Ctx& x, Col<KX, F>& c, const SurfaceIn& s, const Surfa
   w.tsk_gt = w.tskin > w.t2_0;
   w.dthl_v = w.tsk_gt ? vmin(F(p.dtheta), w.tskin - w.t2_0)
                       : vmax(-F(p.dtheta), astab * (w.tskin - w.t2_0));
-  w.denv1 = w.denv0 * (F(1) + w.dthl_v * rdth);
-  const F rhdrag = fdiv(F(1), F(9.81) * F(p.hdrag));
+  w.denv1 = w.denv0 * (F(1) + w.dthl_v * w.rdth);
   const F ph = F(s.phis0) > F(0) ? F(s.phis0) : F(0);
-  w.forog = F(1) + rhdrag * (F(1) - fexp(-ph * rhdrag));
+  w.forog = F(1) + w.rhdrag * (F(1) - fexp(-ph * w.rhdrag));
   w.cdldv = F(p.cdl) * w.denv0 * w.forog;
   w.ustr0 = -w.cdldv * c.u;
   w.vstr0 = -w.cdldv * c.v;
@@ -1302,7 +1316,7 @@ SPD_HD void surface(const Ctx& x, Col<KX, F>& c, const SurfaceIn& s, const Surfa
   w.sst_gt = F(s.sst) > w.t2_1;
   w.dths_v = w.sst_gt ? vmin(F(p.dtheta), F(s.sst) - w.t2_1)
                       : vmax(-F(p.dtheta), astab * (F(s.sst) - w.t2_1));
-  w.denv2 = w.denv0 * (F(1) + w.dths_v * rdth);
+  w.denv2 = w.denv0 * (F(1) + w.dths_v * w.rdth);
   if (fh) w.qs11 = qsat_d(w.t1_1, c.psa, F(1), w.qs11_t, w.qs11_p);
   w.q1_1 = fh ? F(p.fhum0) * (c.RH(KX - 1) * w.qs11) + (F(1) - F(p.fhum0)) * c.q[KX - 1]
               : c.q[KX - 1];
@@ -1340,7 +1354,6 @@ SPD_HD void surface_rev(const Ctx& x, const Col<KX, F>& c, const SurfaceIn& s,
   if (!(x.flags & SPD_LFLUXLAND)) return;  // every flux is a constant zero
   const F esbc = F(p.emisfc) * F(5.67e-8);
   const F astab = (x.flags & SPD_LSCASYM) ? F(0.5) : F(1.0);
-  const F rdth = fdiv(F(p.fstab), F(p.dtheta));
   const F chlcp = F(p.chl) * F(1004.0);
   const F gs = F(vg.grdsig[KX - 1]), gc = F(vg.grdscp[KX - 1]);
   const F rps_b = du_b * w.ustr2 * gs + dv_b * w.vstr2 * gs + dtK_b * w.shf2 * gc +
@@ -1383,10 +1396,10 @@ SPD_HD void surface_rev(const Ctx& x, const Col<KX, F>& c, const SurfaceIn& s,
   } else {
     b.q[KX - 1] += q1_1_b;
   }
-  // denv2 = denv0 (1 + dths rdth)
-  denv0_b += denv2_b * (F(1) + w.dths_v * rdth);
+  // denv2 = denv0 (1 + dths w.rdth)
+  denv0_b += denv2_b * (F(1) + w.dths_v * w.rdth);
   {
-    const F dths_b = denv2_b * w.denv0 * rdth;
+    const F dths_b = denv2_b * w.denv0 * w.rdth;
     if (w.sst_gt)
       t2_1_b -= dths_b * wmin(F(s.sst) - w.t2_1, F(p.dtheta));
     else
@@ -1453,10 +1466,10 @@ SPD_HD void surface_rev(const Ctx& x, const Col<KX, F>& c, const SurfaceIn& s,
     va_b += -vstr0_b * w.cdldv;
     denv0_b += cd_b * F(p.cdl) * w.forog;
   }
-  // denv1 = denv0 (1 + dthl rdth)
-  denv0_b += denv1_b * (F(1) + w.dthl_v * rdth);
+  // denv1 = denv0 (1 + dthl w.rdth)
+  denv0_b += denv1_b * (F(1) + w.dthl_v * w.rdth);
   {
-    const F dthl_b = denv1_b * w.denv0 * rdth;
+    const F dthl_b = denv1_b * w.denv0 * w.rdth;
     F d_b;
     if (w.tsk_gt)
       d_b = dthl_b * wmin(w.tskin - w.t2_0, F(p.dtheta));
@@ -1711,6 +1724,8 @@ SPD_HD void column_vjp(const Ctx& x, const DiffParams<F>& g, F ablco2, F dt_seco
   Lw<KX, F>& lw = sc.lw;
   longwave_down(x, c, ablco2, lw);
   Sf<F> sf;
+  sf.rdth = F(p.fstab) / F(p.dtheta);
+  sf.rhdrag = F(1) / (F(9.81) * F(p.hdrag));
   surface(x, c, s, z, sf);
   longwave_up(x, c, z, ablco2, lw);
   // ---- cotangents of the physics tendencies ----

@@ -364,6 +364,7 @@ __device__ __forceinline__ void column_vjp_smem(const ConstsD& CD, float* sm,
                                                 const VjpMemberDev& m, int c, int Ci,
                                                 bool valid, float* par) {
   using spdvjp::fdiv;
+  using spdvjp::fdiv_full;
   using spdvjp::frcp;
   using spdvjp::wmax;
   using spdvjp::wmin;
@@ -601,6 +602,8 @@ __device__ __forceinline__ void column_vjp_smem(const ConstsD& CD, float* sm,
     const spdvjp::Ctx x{&vg, &p, K.flags, K.model_step, S};
     const spdvjp::SurfaceRow zr{z.fsol, z.ozupp, z.ozone, z.zenit, z.stratz, z.sqrt_coa};
     spdvjp::Sf<float> sf;
+    sf.rdth = D.rdth;
+    sf.rhdrag = D.rhdrag;
     spdvjp::surface<KX, float>(x, cc, sf_in, zr, sf);
     if (verify) {
       const float q_b = Q[B], qs_b1 = QS[B - 1];
@@ -648,7 +651,7 @@ __device__ __forceinline__ void column_vjp_smem(const ConstsD& CD, float* sm,
         } else {
           dq = dq + 0.0f;
         }
-        if (oro) dq = dq + fdiv(qcorh * D.qcorv[k], dts);
+        if (oro) dq = dq + fdiv_full(qcorh * D.qcorv[k], dts);
         TB[k] = dq;
       }
       // the humidity as given, read again where it was clamped, all levels' loads first
@@ -909,7 +912,7 @@ __device__ __forceinline__ void column_vjp_smem(const ConstsD& CD, float* sm,
     const float phiB = col.at(col.phi, B), phin = col.at(col.phi, nl1);
     const float seB = kCp * T[B] + phiB, sen = kCp * T[nl1] + phin;
     const float den = phin - phiB;
-    const float rden = frcp(den), gse = (sen - seB) * rden;
+    const float rden = frcp(den), gse = fdiv_full(sen - seB, den);  // den may be zero
     const float rrcl = D.rrcl;
     const float pr1v = 86.4f * (o.precnv + o.precls);
     const float pr1 = spdvjp::vmin(p.pmaxcl, pr1v);
@@ -1293,7 +1296,7 @@ __device__ __forceinline__ void column_vjp_smem(const ConstsD& CD, float* sm,
           psa_b += fmaf(fpsa_b, mn2, y_b * D.rdps);
           par[spdvjp::P_PSMIN] +=
               y_b * (psa - p.psmin) * (0.5f * D.rdps * D.rdps) - y_b * D.rdps;
-          par[spdvjp::P_TRCNV] += -(A_b * fpsa) * fdiv(D.fm0, p.trcnv);
+          par[spdvjp::P_TRCNV] += -(A_b * fpsa) * D.fm0_t;
           qb3_b = qb_b * wmin(qb3, q_B);
           qk_b = fmaf(qb_b, wmin(q_B, qb3), qk_b);
           sb3_b = fds_b * fmass;
@@ -1413,7 +1416,7 @@ __device__ __forceinline__ void column_vjp_smem(const ConstsD& CD, float* sm,
         const size_t i = k * C;
         const float qk = ((neg >> k) & 1u) ? 0.0f : q_b;
         __stcs(gt + i, tb);
-        __stcs(gq + i, qk + (lim ? -fdiv(ctq, rdt) : 0.0f));
+        __stcs(gq + i, qk + (lim ? -fdiv_full(ctq, rdt) : 0.0f));
         __stcs(gp + i, PB[k]);
         if (k < B) {
           __stcs(gu + i, 0.0f);
@@ -1421,7 +1424,7 @@ __device__ __forceinline__ void column_vjp_smem(const ConstsD& CD, float* sm,
         }
       }
     }
-    par[spdvjp::P_TRLSC] += -rtlsc_b * fdiv(D.rtlsc, p.trlsc);
+    par[spdvjp::P_TRLSC] += -rtlsc_b * D.rtlsc_t;
     psa_b = fmaf(psa2_b, 2.0f * psa, psa_b);
     psa_b -= (xps + dps) * rpsa;
     if (valid) {

@@ -1,5 +1,7 @@
-"""The device adjoint where a parameter stands at an end of its range: entrainment off
-(entmax = 0), against the host builds of the hand-written reverse pass.
+"""The device adjoint where a parameter or a field stands at an end of its range: entrainment off
+(entmax = 0), a process switched off by an infinite time or scale, equal geopotentials at the two
+lowest levels (an infinite gradient of the dry static energy), against the host builds of the
+hand-written reverse pass; and its division against IEEE division.
 
 The bar is that of tests/test_adjoint_tiles_gpu.py: each gradient plane within 1e-4 of its largest
 value, or three times the host float32 build's own distance from float64; each parameter's sum
@@ -68,9 +70,11 @@ def check(pkg, host, inst, **values):
                     want[m][n][at] = g[n][0]
     w64, w32 = (want[m] for m in modes)
     for n, v in got.items():
-        scale = max(np.abs(w64[n]).max(), 1e-30)
-        tol = max(1e-4, 3 * np.abs(w32[n] - w64[n]).max() / scale)
-        err = np.abs(v - w64[n]).max() / scale
+        ok = np.isfinite(w64[n])
+        assert np.array_equal(np.isfinite(v), ok), (values, n)
+        scale = max(np.abs(w64[n][ok]).max(), 1e-30)
+        tol = max(1e-4, 3 * np.abs(w32[n][ok] - w64[n][ok]).max() / scale)
+        err = np.abs(v[ok] - w64[n][ok]).max() / scale
         assert err <= tol, (values, n, err, tol)
     p64, p32 = (par[m] for m in modes)
     total = p64.sum(0)
@@ -84,3 +88,67 @@ def test_no_entrainment(pkg, host, kx):
     inst = pkg.synthetic.land_instance(31 * kx + 43, 43, 3, kx)
     gp = check(pkg, host, inst, convection__entmax=0.0)
     assert gp[4] != 0.0  # the derivative at zero is one-sided and finite
+
+
+@pytest.mark.parametrize("kx", [7, 8, 16])
+@pytest.mark.parametrize("name", ["convection__trcnv", "condensation__trlsc",
+                                  "surface_flux__hdrag"])
+def test_process_switched_off(pkg, host, kx, name):
+    inst = pkg.synthetic.land_instance(31 * kx + 43, 43, 3, kx)
+    check(pkg, host, inst, **{name: float("inf")})
+
+
+@pytest.mark.parametrize("kx", [7, 8, 16])
+def test_equal_lowest_geopotentials(pkg, host, kx):
+    inst = pkg.synthetic.land_instance(31 * kx + 43, 43, 3, kx)
+    inst.phi[-2] = inst.phi[-1]
+    check(pkg, host, inst)
+
+
+def divide(pkg, a, b):
+    """The device's a / b, 1 / b and a / b by the full form, and IEEE's a / b and 1 / b."""
+    import ctypes as C
+    import torch
+    on = lambda x: torch.as_tensor(x, dtype=torch.float32, device="cuda")
+    x, y, out = on(a), on(b), torch.empty(3, len(a), device="cuda")
+    p = lambda t: C.c_void_p(t.data_ptr())
+    rc = pkg._lib.load().spd_selftest_division(
+        len(a), p(x), p(y), p(out), C.c_void_p(torch.cuda.current_stream().cuda_stream))
+    assert rc == 0
+    with np.errstate(all="ignore"):
+        return (*out.cpu().numpy(), a / b, np.float32(1) / b)
+
+
+def test_division_rounds_like_ieee(pkg):
+    """Operands and quotients far from the ends of the exponent range.  The residual of a quotient
+    within an ulp is exact, so the corrected one is within half an ulp and a little: never more
+    than an ulp from IEEE's, and other than IEEE's only where that little decides (at most one in
+    a million is asked for).  The reciprocal has one rounding after its Newton step: one ulp.
+    The full form gives the same bits here."""
+    rng = np.random.default_rng(20261205)
+    n = 1 << 24
+    draw = lambda: (rng.uniform(1.0, 2.0, n) * np.exp2(rng.integers(-40, 41, n))
+                    * rng.choice([-1.0, 1.0], n)).astype(np.float32)
+    short, r, full, q0, r0 = divide(pkg, draw(), draw())
+    assert np.array_equal(short.view(np.int32), full.view(np.int32))
+    ulps = lambda x, y: np.abs(x.view(np.int32).astype(np.int64) - y.view(np.int32))
+    assert ulps(r, r0).max() <= 1
+    d = ulps(short, q0)
+    assert d.max() <= 1 and (d != 0).sum() <= n // 1000000, (d.max(), (d != 0).sum())
+
+
+def test_division_at_the_ends(pkg):
+    """The full form on every pair of zeros, infinities, NaN and finite values up to 2^125 in size:
+    IEEE's result, but for an ulp of a subnormal one; and the two exceptions, a subnormal divisor
+    (counts as zero) and one above 2^126 (counts as infinite)."""
+    f = np.float32
+    size = np.array([0.0, np.inf, np.nan, 1.0, 3.0, 1e-30, 1e30, 2.0 ** -126, 2.0 ** 125], f)
+    e = np.concatenate([size, -size])
+    a, b = (x.ravel().copy() for x in np.meshgrid(e, e))
+    _, _, got, want, _ = divide(pkg, a, b)
+    same = (got == want) | (np.isnan(got) & np.isnan(want))
+    with np.errstate(invalid="ignore"):
+        same |= np.abs(got.astype(float) - want.astype(float)) <= 2.0 ** -149
+    assert same.all(), [t for t, s in zip(zip(a, b, got, want), same) if not s]
+    x, y = np.array([1.0, 1.0, 1e-39, 2.0 ** 127], f), np.array([1e-39, 2.0 ** 127] * 2, f)
+    assert np.array_equal(divide(pkg, x, y)[2], np.array([np.inf, 0.0, np.inf, 0.0], f))
