@@ -44,14 +44,16 @@ class HeldSuarezPhysics(Physics):
 
     def _lat_table(self, geometry: Geometry, device):
         """sin^2, cos^2, cos^4 of the latitudes, formed in float32 as the reference does
-        (held_suarez_physics.py:58-61, :72-73), on the device (cached per geometry)."""
-        key = (id(geometry), str(device))
+        (held_suarez_physics.py:58-61, :72-73), on the device.  Kept by the latitudes' values, and
+        never dropped: a kernel on another stream may still read it."""
+        lat = np.asarray(geometry.radang, np.float64)
+        key = (lat.tobytes(), str(device))
         tab = self._tables.get(key)
         if tab is None:
-            la = np.asarray(geometry.radang, np.float64).astype(np.float32)
+            la = lat.astype(np.float32)
             host = np.stack([np.sin(la) ** 2, np.cos(la) ** 2, np.cos(la) ** 4]).astype(np.float32)
             tab = torch.as_tensor(host, device=device).contiguous()
-            self._tables = {key: tab}
+            self._tables[key] = tab
         return tab
 
     def compute_tendencies(self, state: PhysicsState, forcing=None,
