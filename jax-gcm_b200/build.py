@@ -80,7 +80,11 @@ def calls_command():
             "-I" + os.path.join(inc, "torch", "csrc", "api", "include"),
             "-I" + sysconfig.get_paths()["include"], "-I" + os.path.join(cuda, "include"),
             os.path.join(HERE, CALLS_SOURCE), "-o", calls_path(), "-L" + lib, "-ltorch_python",
-            "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda"]
+            "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda",
+            # the C++ runtime that torch runs on, by its name: where g++'s own libstdc++.so is
+            # missing, -lstdc++ takes the archive, and the first exception in the module's private
+            # copy ends the interpreter
+            "-nostdlib++", "-l:libstdc++.so.6"]
 
 
 def needs_calls():
