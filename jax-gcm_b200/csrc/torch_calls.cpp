@@ -48,7 +48,28 @@ Name g_inputs[] = {{"u_wind", kState, nullptr}, {"v_wind", kState, nullptr},
 constexpr int kInputs = sizeof(g_inputs) / sizeof(g_inputs[0]);
 static_assert(kInputs * sizeof(void*) == sizeof(spd_inputs_t), "one pointer per input field");
 constexpr int kOutputs = sizeof(spd_outputs_t) / sizeof(void*);
+constexpr int kLevelInputs = 5, kLatitudeInputs = 2;  // the first ones, and the last
+const char* const g_outputs[] = {"u_wind", "v_wind", "temperature", "specific_humidity", "precnv",
+                                 "precls", "cbmf", "cloudc", "cloudstr", "rsds", "rsns", "ftop_sw",
+                                 "rlds", "rlns", "ftop_lw", "tsfc", "tskin", "shf", "evap",
+                                 "iptop", "icltop"};
+static_assert(sizeof(g_outputs) / sizeof(g_outputs[0]) == kOutputs, "one name per output field");
 constexpr int kLevelOutputs = 4, kFloatOutputs = 19, kPlainOutputs = 6;
+
+// The kernels' extents come from the geometry, not from the tensors: a field has to hold the values
+// that they read, and a result the bytes that they write.
+void expect_values(const at::Tensor& t, int64_t need, const char* name) {
+  TORCH_CHECK_VALUE(t.numel() >= need, name, " has ", t.numel(), " values, the geometry has ", need);
+}
+void expect_room(const at::Tensor& t, int64_t need, const char* name) {
+  const int64_t room =
+      (int64_t)t.storage().nbytes() - t.storage_offset() * (int64_t)t.element_size();
+  TORCH_CHECK_VALUE(room >= need * 4, name, " (out) has room for ", room / 4,
+                    " values, the geometry has ", need);
+}
+void expect_device(const at::Tensor& t) {
+  TORCH_CHECK(t.is_cuda() || t.is_pinned(), "out holds CUDA tensors");
+}
 
 at::Tensor attribute(PyObject* obj, PyObject* name) {
   PyObject* v = PyObject_GetAttr(obj, name);
@@ -76,12 +97,20 @@ struct Fields {
   spd_inputs_t in;
 };
 
-Fields fields(PyObject* state, PyObject* forcing, PyObject* geometry, c10::Device device) {
+// low_winds: u and v are planes of the lowest level.
+Fields fields(PyObject* state, PyObject* forcing, PyObject* geometry, c10::Device device,
+              const spd_desc_t* desc, bool low_winds) {
+  const int64_t columns = (int64_t)desc->ix * desc->il, level = desc->kx * columns;
   PyObject* const owners[] = {state, forcing, geometry};
   Fields f;
   const float** p = reinterpret_cast<const float**>(&f.in);
   for (int i = 0; i < kInputs; ++i) {
-    f.t[i] = as_input(attribute(owners[g_inputs[i].owner], g_inputs[i].str), device);
+    at::Tensor t = attribute(owners[g_inputs[i].owner], g_inputs[i].str);
+    expect_values(t, i >= kInputs - kLatitudeInputs                       ? desc->il
+                     : i < kLevelInputs && !(low_winds && i < 2) ? level
+                                                                 : columns,
+                  g_inputs[i].text);
+    f.t[i] = as_input(std::move(t), device);
     p[i] = static_cast<const float*>(f.t[i].const_data_ptr());
   }
   return f;
@@ -125,27 +154,35 @@ PyObject* fwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
   expect(n, 11);
   const auto* desc = address<const spd_desc_t>(a[5]);
   const c10::Device device = device_of(a[0]);
-  Fields f = fields(a[0], a[1], a[2], device);
+  const bool low_winds = (desc->flags & SPD_LOW_LEVEL_WINDS) != 0;
+  Fields f = fields(a[0], a[1], a[2], device, desc, low_winds);
+  const int64_t columns = (int64_t)desc->ix * desc->il;
   std::array<at::Tensor, kOutputs> t;
   spd_outputs_t out{};
   void** p = reinterpret_cast<void**>(&out);
-  if (a[3] == Py_None) {
-    const int64_t level[] = {desc->kx, desc->ix, desc->il}, surface[] = {desc->ix, desc->il};
-    const int count = PyObject_IsTrue(a[4]) == 1 ? kOutputs : kPlainOutputs;
-    for (int i = 0; i < count; ++i) {
-      t[i] = i < kLevelOutputs ? empty(level, device)
-                               : empty(surface, device, i < kFloatOutputs ? at::kFloat : at::kInt);
-      p[i] = t[i].data_ptr();
-    }
-  } else {
+  if (a[3] != Py_None) {
     TORCH_CHECK_TYPE(PyList_Check(a[3]) && PyList_GET_SIZE(a[3]) == kOutputs, "out is a list");
     for (int i = 0; i < kOutputs; ++i) {
       PyObject* v = PyList_GET_ITEM(a[3], i);
       if (v == Py_None) continue;
       TORCH_CHECK_TYPE(THPVariable_Check(v), "out holds tensors");
       t[i] = THPVariable_Unpack(v);
-      p[i] = t[i].data_ptr();
+      expect_room(t[i], i < kLevelOutputs && !(low_winds && i < 2) ? desc->kx * columns : columns,
+                  g_outputs[i]);
     }
+  }
+  TORCH_CHECK(device.is_cuda(), "the physics runs on CUDA tensors only (no CPU path)");
+  if (a[3] == Py_None) {
+    const int64_t level[] = {desc->kx, desc->ix, desc->il}, surface[] = {desc->ix, desc->il};
+    const int count = PyObject_IsTrue(a[4]) == 1 ? kOutputs : kPlainOutputs;
+    for (int i = 0; i < count; ++i)
+      t[i] = i < kLevelOutputs ? empty(level, device)
+                               : empty(surface, device, i < kFloatOutputs ? at::kFloat : at::kInt);
+  }
+  for (int i = 0; i < kOutputs; ++i) {
+    if (!t[i].defined()) continue;
+    expect_device(t[i]);
+    p[i] = t[i].data_ptr();
   }
   void* stream = stream_of(device);
   const auto* vgrid = address<const spd_vgrid_t>(a[6]);
@@ -167,16 +204,19 @@ PyObject* fwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
 PyObject* vjp(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   expect(n, 9);
+  const auto* desc = address<const spd_desc_t>(a[4]);
   const c10::Device device = device_of(a[0]);
-  TORCH_CHECK(device.is_cuda(), "the adjoint runs on CUDA tensors only (no CPU path)");
-  Fields f = fields(a[0], a[1], a[2], device);
+  Fields f = fields(a[0], a[1], a[2], device, desc, false);
   std::array<at::Tensor, 4> ct;
   spd_cotangents_t cot;
   const float** pc = reinterpret_cast<const float**>(&cot);
   for (int i = 0; i < 4; ++i) {
-    ct[i] = as_input(attribute(a[3], g_inputs[i].str), device);
+    at::Tensor t = attribute(a[3], g_inputs[i].str);
+    expect_values(t, (int64_t)desc->kx * desc->ix * desc->il, g_inputs[i].text);
+    ct[i] = as_input(std::move(t), device);
     pc[i] = static_cast<const float*>(ct[i].const_data_ptr());
   }
+  TORCH_CHECK(device.is_cuda(), "the adjoint runs on CUDA tensors only (no CPU path)");
   std::array<at::Tensor, 7> g;
   spd_grads_t grads;
   float** pg = reinterpret_cast<float**>(&grads);
@@ -185,7 +225,6 @@ PyObject* vjp(PyObject*, PyObject* const* a, Py_ssize_t n) {
     pg[i] = static_cast<float*>(g[i].data_ptr());
   }
   void* stream = stream_of(device);
-  const auto* desc = address<const spd_desc_t>(a[4]);
   const auto* vgrid = address<const spd_vgrid_t>(a[5]);
   const auto* params = address<const spd_params_t>(a[6]);
   void* scratch = address<void>(a[7]);
@@ -204,22 +243,32 @@ PyObject* held_suarez(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   expect(n, 4);
   const c10::Device device = device_of(a[0]);
+  const auto* desc = address<const spd_hs_desc_t>(a[3]);
+  const int64_t columns = (int64_t)desc->ix * desc->il, level = desc->kx * columns;
   const int which[] = {0, 1, 2, 5};  // u, v, T, psa
   std::array<at::Tensor, 4> in, out;
-  for (int i = 0; i < 4; ++i) in[i] = as_input(attribute(a[0], g_inputs[which[i]].str), device);
+  for (int i = 0; i < 4; ++i) {
+    at::Tensor t = attribute(a[0], g_inputs[which[i]].str);
+    expect_values(t, i < 3 ? level : columns, g_inputs[which[i]].text);
+    in[i] = as_input(std::move(t), device);
+  }
   TORCH_CHECK_TYPE(THPVariable_Check(a[1]), "the latitude table is a tensor");
   const at::Tensor& table = THPVariable_Unpack(a[1]);
-  for (int i = 0; i < 4; ++i) {
-    if (a[2] == Py_None) {
-      out[i] = empty(in[2].sizes(), device);
-    } else {
-      TORCH_CHECK_TYPE(PyList_Check(a[2]) && PyList_GET_SIZE(a[2]) == 4, "out is a list of four");
-      PyObject* v = PyList_GET_ITEM(a[2], i);
-      TORCH_CHECK_TYPE(THPVariable_Check(v), "out holds tensors");
-      out[i] = THPVariable_Unpack(v);
-    }
+  TORCH_CHECK_VALUE(table.numel() == 3 * (int64_t)desc->il && table.is_contiguous() &&
+                        table.scalar_type() == at::kFloat && table.device() == device,
+                    "the latitude table has three values for each of the geometry's latitudes");
+  for (int i = 0; i < 4 && a[2] != Py_None; ++i) {
+    TORCH_CHECK_TYPE(PyList_Check(a[2]) && PyList_GET_SIZE(a[2]) == 4, "out is a list of four");
+    PyObject* v = PyList_GET_ITEM(a[2], i);
+    TORCH_CHECK_TYPE(THPVariable_Check(v), "out holds tensors");
+    out[i] = THPVariable_Unpack(v);
+    expect_room(out[i], level, g_outputs[i]);
   }
-  const auto* desc = address<const spd_hs_desc_t>(a[3]);
+  TORCH_CHECK(device.is_cuda(), "HeldSuarezPhysics runs on CUDA tensors only (no CPU path)");
+  for (at::Tensor& t : out) {
+    if (!t.defined()) t = empty(in[2].sizes(), device);
+    expect_device(t);
+  }
   void* stream = stream_of(device);
   auto p = [](const at::Tensor& t) { return static_cast<const float*>(t.const_data_ptr()); };
   auto w = [](const at::Tensor& t) { return static_cast<float*>(t.data_ptr()); };
