@@ -29,7 +29,7 @@ class HeldSuarezPhysics(Physics):
                  dTy: float = 60.0, dThz: float = 10.0, kappa: float = 2.0 / 7.0):
         self.sigma_b, self.kf, self.ka, self.ks = sigma_b, kf, ka, ks
         self.minT, self.maxT, self.dTy, self.dThz, self.kappa = minT, maxT, dTy, dThz, kappa
-        self._tables = {}
+        self._tables = []  # (latitudes, device, table)
 
     def _desc(self, geometry: Geometry):
         kx, ix, il = geometry.nodal_shape
@@ -47,13 +47,14 @@ class HeldSuarezPhysics(Physics):
         (held_suarez_physics.py:58-61, :72-73), on the device.  Kept by the latitudes' values, and
         never dropped: a kernel on another stream may still read it."""
         lat = np.asarray(geometry.radang, np.float64)
-        key = (lat.tobytes(), str(device))
-        tab = self._tables.get(key)
-        if tab is None:
-            la = lat.astype(np.float32)
-            host = np.stack([np.sin(la) ** 2, np.cos(la) ** 2, np.cos(la) ** 4]).astype(np.float32)
-            tab = torch.as_tensor(host, device=device).contiguous()
-            self._tables[key] = tab
+        key = lat.tobytes()
+        for values, dev, tab in self._tables:  # comparing is cheaper than hashing, and these are few
+            if dev == device and values == key:
+                return tab
+        la = lat.astype(np.float32)
+        host = np.stack([np.sin(la) ** 2, np.cos(la) ** 2, np.cos(la) ** 4]).astype(np.float32)
+        tab = torch.as_tensor(host, device=device).contiguous()
+        self._tables.append((key, device, tab))
         return tab
 
     def compute_tendencies(self, state: PhysicsState, forcing=None,
