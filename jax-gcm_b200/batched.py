@@ -92,12 +92,25 @@ class Ensemble:
             for k in ("u_wind", "v_wind"):
                 if tensors[k].numel() != wind_numel:
                     raise ValueError(f"member {i}: {k} must have {wind_numel} elements")
+            # the kernels' extents come from the geometry
+            need = {k: ix * il for k in _lib.INPUT_FIELDS + _lib.OUTPUT_FIELDS}
+            need.update(u_wind=wind_numel, v_wind=wind_numel, sia=il, coa=il)
+            need.update(dict.fromkeys(("temperature", "specific_humidity", "geopotential"),
+                                      kx * ix * il))
+            for k, v in tensors.items():
+                if v.numel() < need[k]:
+                    raise ValueError(f"member {i}: {k} must have {need[k]} elements")
             if m.out is None:
                 e3 = lambda: torch.empty((kx, ix, il), dtype=torch.float32, device=dev)
                 e2 = lambda: torch.empty((ix, il), dtype=torch.float32, device=dev)
                 ew = e2 if low_level_winds else e3
                 m.out = dict(u_wind=ew(), v_wind=ew(), temperature=e3(), specific_humidity=e3(),
                              precnv=e2(), precls=e2())
+            for k in _lib.OUTPUT_FIELDS:
+                v = m.out.get(k)
+                if v is not None and (v.untyped_storage().nbytes()
+                                      - v.storage_offset() * v.element_size()) < 4 * need[k]:
+                    raise ValueError(f"member {i}: out {k} must have {need[k]} elements")
             mem[i].inp = _lib.Inputs(**{k: tensors[k].data_ptr() for k in _lib.INPUT_FIELDS})
             mem[i].out = _lib.Outputs(**{k: (m.out[k].data_ptr() if k in m.out else None)
                                          for k in _lib.OUTPUT_FIELDS})

@@ -121,3 +121,25 @@ def test_held_suarez(calls, name):
         setattr(st, name, short(getattr(st, name)))
     with pytest.raises(ValueError):
         calls.held_suarez(st, tab, out, C.addressof(d))
+
+
+@pytest.mark.parametrize("name", STATE + SURFACE + ("fmask", "orog", "phis0", "sia", "coa"))
+def test_short_ensemble_inputs(monkeypatch, name):
+    monkeypatch.setattr(L, "preload", lambda index: None)
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 0)
+    st, fo, ge, da = objects()
+    owner = next(o for o in (st, fo, ge) if hasattr(o, name))
+    setattr(owner, name, short(getattr(owner, name)))
+    with pytest.raises(ValueError, match=name):
+        pkg.Ensemble([pkg.Member(st, fo, ge)], da)
+
+
+@pytest.mark.parametrize("name", TENDENCY + ("precnv", "rsds", "icltop"))
+def test_short_ensemble_outputs(monkeypatch, name):
+    monkeypatch.setattr(L, "preload", lambda index: None)
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 0)
+    st, fo, ge, da = objects()
+    out = {f: torch.zeros((KX, IX, IL) if f in TENDENCY else (IX, IL)) for f in L.OUTPUT_FIELDS}
+    out[name] = short(out[name]).clone()
+    with pytest.raises(ValueError, match=name):
+        pkg.Ensemble([pkg.Member(st, fo, ge, out)], da)
