@@ -26,17 +26,6 @@ DIFF_PARAMS = [("convection", "psmin"), ("convection", "trcnv"), ("convection", 
                ("condensation", "drhlsc"), ("condensation", "rhblsc"),
                ("shortwave_radiation", "albcl"), ("shortwave_radiation", "albcls")]
 
-_SCRATCH = {}
-
-
-def _scratch(nbytes, device):
-    key = (str(device),)
-    buf = _SCRATCH.get(key)
-    if buf is None or buf.numel() < nbytes:
-        buf = torch.empty(nbytes, dtype=torch.uint8, device=device)
-        _SCRATCH[key] = buf
-    return buf
-
 
 def vjp(physics: SpeedyPhysics, state: PhysicsState, forcing, geometry, date,
         cotangent: PhysicsTendency):
@@ -47,11 +36,9 @@ def vjp(physics: SpeedyPhysics, state: PhysicsState, forcing, geometry, date,
     _lib.preload(dev.index if dev.index is not None else torch.cuda.current_device())
     f2 = forcing.day_slice(date.model_day())
     desc = physics.desc(geometry, date, forcing.lfluxland)
-    n = lib.spd_vjp_scratch_bytes(C.byref(desc))
-    sc = _scratch(n, dev)
     rc, g = calls.vjp(state, f2, geometry, cotangent, C.addressof(desc),
-                      C.addressof(geometry.vgrid()), C.addressof(physics._pstruct), sc.data_ptr(),
-                      n)
+                      C.addressof(geometry.vgrid()), C.addressof(physics._pstruct),
+                      lib.spd_vjp_scratch_bytes(C.byref(desc)))
     _lib.check(rc, "spd_vjp")
     return PhysicsState(*g[:6]), g[6]
 

@@ -199,11 +199,13 @@ PyObject* fwd(PyObject*, PyObject* const* a, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
-// vjp(state, forcing, geometry, cotangent, desc, vgrid, params, scratch, scratch_bytes)
+// vjp(state, forcing, geometry, cotangent, desc, vgrid, params, scratch_bytes)
 //   -> (status, [u, v, T, q, phi, psa, params gradients])
+// The scratch is the call's own, from torch's allocator on the current stream: calls on several
+// streams or from several threads do not meet in it.
 PyObject* vjp(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
-  expect(n, 9);
+  expect(n, 8);
   const auto* desc = address<const spd_desc_t>(a[4]);
   const c10::Device device = device_of(a[0]);
   Fields f = fields(a[0], a[1], a[2], device, desc, false);
@@ -227,8 +229,10 @@ PyObject* vjp(PyObject*, PyObject* const* a, Py_ssize_t n) {
   void* stream = stream_of(device);
   const auto* vgrid = address<const spd_vgrid_t>(a[5]);
   const auto* params = address<const spd_params_t>(a[6]);
-  void* scratch = address<void>(a[7]);
-  const size_t bytes = PyLong_AsSize_t(a[8]);
+  const size_t bytes = PyLong_AsSize_t(a[7]);
+  if (PyErr_Occurred()) throw python_error();
+  const at::Tensor own = empty({(int64_t)bytes}, device, at::kByte);
+  void* scratch = own.data_ptr();
   int rc;
   {
     pybind11::gil_scoped_release release;

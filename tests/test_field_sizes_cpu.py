@@ -42,7 +42,7 @@ def vjp(calls, st, fo, ge, da, ct):
     phys = pkg.SpeedyPhysics()
     keep, (d, vg, p) = arguments(phys, ge, da, fo)
     n = L.load().spd_vjp_scratch_bytes(C.byref(keep[0]))
-    return calls.vjp(st, fo, ge, ct, d, vg, p, 256, n)
+    return calls.vjp(st, fo, ge, ct, d, vg, p, n)
 
 
 def short(t):

@@ -25,7 +25,7 @@ for name in ("fwd", "vjp", "held_suarez", "rollout_step", "rollout_reverse", "bi
 st, fo, ge, da = pkg.instance_to_device(inst, "cpu")
 st.temperature = 3
 error("fwd", st, fo, ge, None, True, 64, 64, 64, 64, 64, 0)
-error("vjp", st, fo, ge, st, 64, 64, 64, 64, 64)
+error("vjp", st, fo, ge, st, 64, 64, 64, 64)
 error("held_suarez", st, st.u_wind, None, 64)
 del st.u_wind
 error("rollout_step", st, st, 1.0)

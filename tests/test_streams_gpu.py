@@ -1,0 +1,49 @@
+"""Calls that overlap on two streams give the bits of the same calls one after the other."""
+import importlib
+from dataclasses import replace
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+STATE = ("u_wind", "v_wind", "temperature", "specific_humidity", "geopotential",
+         "normalized_surface_pressure")
+
+
+@pytest.fixture(scope="module")
+def pkg():
+    return importlib.import_module("jax-gcm_b200")
+
+
+def instances(pkg):
+    """Two instances of one size whose dates, solar rows and level sets differ."""
+    import torch
+    out = []
+    for i in range(2):
+        inst = pkg.synthetic.land_instance(40 + i, 96, 48, 8)
+        if i:
+            inst.q[:5, ::7] *= 5.0
+        st, fo, ge, da = pkg.instance_to_device(inst, "cuda")
+        gen = torch.Generator(device="cuda").manual_seed(i)
+        ct = pkg.PhysicsTendency(*(torch.randn(8, 96, 48, generator=gen, device="cuda")
+                                   for _ in range(4)))
+        out.append((st, fo, ge, replace(da, tyear=0.1 + 0.5 * i), ct))
+    return out
+
+
+def test_vjps_on_two_streams(pkg):
+    import torch
+    phys = pkg.SpeedyPhysics(diagnostics=False)
+    cases = instances(pkg)
+    call = lambda c: pkg.adjoint.vjp(phys, *c)[0]
+    want = [call(c) for c in cases]
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in cases]
+    got = []
+    for _ in range(20):
+        for c, s in zip(cases, streams):
+            with torch.cuda.stream(s):
+                got.append(call(c))
+    torch.cuda.synchronize()
+    for i, g in enumerate(got):
+        for n in STATE:
+            assert torch.equal(getattr(g, n), getattr(want[i % 2], n)), (i, n)
