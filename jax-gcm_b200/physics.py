@@ -19,6 +19,7 @@ from __future__ import annotations
 import ctypes as C
 import math
 from dataclasses import dataclass, field, fields, replace
+from threading import get_ident
 from types import SimpleNamespace
 from typing import Optional
 
@@ -427,6 +428,13 @@ def physics_data_from_diagnostics(d):
     )
 
 
+def current_raw_stream(device_index):
+    """The current CUDA stream of a device as a raw handle (torch's own fast path where it has
+    one; torch.cuda.current_stream otherwise)."""
+    f = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+    return f(device_index) if f is not None else torch.cuda.current_stream(device_index).cuda_stream
+
+
 class SpeedyPhysics(Physics):
     """SPEEDY physics on the B200 (speedy_physics.py:34-132).
 
@@ -444,7 +452,8 @@ class SpeedyPhysics(Physics):
     and checks it on the device: the physics runs in one pass over the columns, and a second
     pass follows only when the prediction missed (the first call, or after another instance's
     call).  ``speculate=False`` forms the level set first in a light launch.  Both give the same
-    results bitwise.  Calls of one object use one scratch buffer: order them on one stream.
+    results bitwise.  The prediction is the previous call's on the same stream from the same
+    thread, each of which has a scratch buffer of its own (256 bytes).
     """
 
     def __init__(self, parameters: Optional[Parameters] = None, checkpoint_terms=True,
@@ -484,11 +493,12 @@ class SpeedyPhysics(Physics):
     def _scratch_for(self, desc, device):
         lib = _lib.load()
         n = lib.spd_fwd_scratch_bytes(C.byref(desc))
-        key = (device, n)
+        # The launches of two calls on one scratch must not interleave.  None is dropped while the
+        # object lives: a captured graph may hold its address.
+        key = (device, n, current_raw_stream(device.index), get_ident())
         buf = self._scratch.get(key)
         if buf is None:
-            buf = torch.empty(n, dtype=torch.uint8, device=device)
-            self._scratch = {key: buf}
+            buf = self._scratch[key] = torch.empty(n, dtype=torch.uint8, device=device)
         return buf
 
     def compute_tendencies(self, state: PhysicsState, forcing: ForcingData, geometry: Geometry,
@@ -511,9 +521,10 @@ class SpeedyPhysics(Physics):
         if not t.is_cuda:
             raise RuntimeError("SpeedyPhysics runs on CUDA tensors only (no CPU path)")
         _lib.preload(t.get_device())
-        if self._day[0] != date.tyear:
-            self._day = (date.tyear, date.model_day())
-        f2 = forcing.day_slice(self._day[1])
+        day = self._day
+        if day[0] != date.tyear:
+            day = self._day = (date.tyear, date.model_day())
+        f2 = forcing.day_slice(day[1])
         desc = self.desc(geometry, date, forcing.lfluxland)
         if accumulate:
             desc.flags |= _lib.SPD_ACCUMULATE_DIAGNOSTICS

@@ -47,3 +47,47 @@ def test_vjps_on_two_streams(pkg):
     for i, g in enumerate(got):
         for n in STATE:
             assert torch.equal(getattr(g, n), getattr(want[i % 2], n)), (i, n)
+
+
+def test_forwards_of_one_object_on_two_streams(pkg):
+    import torch
+    cases = [c[:4] for c in instances(pkg)]
+    out = lambda r: [getattr(r[0], n) for n in STATE[:4]] + [r[1].condensation.precls]
+    want = [out(pkg.SpeedyPhysics(speculate=False).compute_tendencies(*c)) for c in cases]
+    torch.cuda.synchronize()
+    phys = pkg.SpeedyPhysics()
+    streams = [torch.cuda.Stream() for _ in cases]
+    got = []
+    for _ in range(20):
+        for c, s in zip(cases, streams):
+            with torch.cuda.stream(s):
+                got.append(out(phys.compute_tendencies(*c)))
+    torch.cuda.synchronize()
+    for i, g in enumerate(got):
+        assert all(torch.equal(a, b) for a, b in zip(g, want[i % 2])), i
+
+
+def test_forwards_of_one_object_from_two_threads(pkg):
+    """Two threads on one stream, whose calls' launches may interleave."""
+    import threading
+
+    import torch
+    cases = [c[:4] for c in instances(pkg)]
+    out = lambda r: [getattr(r[0], n) for n in STATE[:4]] + [r[1].condensation.precls]
+    want = [out(pkg.SpeedyPhysics(speculate=False).compute_tendencies(*c)) for c in cases]
+    phys, got = pkg.SpeedyPhysics(), [[], []]
+
+    def work(i):
+        for _ in range(50):
+            got[i].append(out(phys.compute_tendencies(*cases[i])))
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    for i in range(2):
+        assert len(got[i]) == 50
+        for g in got[i]:
+            assert all(torch.equal(a, b) for a, b in zip(g, want[i])), i
