@@ -36,9 +36,9 @@ def vjp(physics: SpeedyPhysics, state: PhysicsState, forcing, geometry, date,
     _lib.preload(dev.index if dev.index is not None else torch.cuda.current_device())
     f2 = forcing.day_slice(date.model_day())
     desc = physics.desc(geometry, date, forcing.lfluxland)
-    rc, g = calls.vjp(state, f2, geometry, cotangent, C.addressof(desc),
-                      C.addressof(geometry.vgrid()), C.addressof(physics._pstruct),
-                      lib.spd_vjp_scratch_bytes(C.byref(desc)))
+    vgrid, params = geometry.vgrid(), physics._pstruct  # held until the call returns
+    rc, g = calls.vjp(state, f2, geometry, cotangent, C.addressof(desc), C.addressof(vgrid),
+                      C.addressof(params), lib.spd_vjp_scratch_bytes(C.byref(desc)))
     _lib.check(rc, "spd_vjp")
     return PhysicsState(*g[:6]), g[6]
 

@@ -529,11 +529,11 @@ class SpeedyPhysics(Physics):
         if accumulate:
             desc.flags |= _lib.SPD_ACCUMULATE_DIAGNOSTICS
         scratch = self._scratch_for(desc, t.device)
+        vgrid, params = geometry.vgrid(), self._pstruct  # held until the call returns
         given = None if out is None else [out.get(k) for k in _lib.OUTPUT_FIELDS]
         rc, outs = calls.fwd(state, f2, geometry, given, self.diagnostics, C.addressof(desc),
-                             C.addressof(geometry.vgrid()), C.addressof(self._pstruct),
-                             scratch.data_ptr(), scratch.numel(),
-                             0 if marker is None else marker.cuda_event)
+                             C.addressof(vgrid), C.addressof(params), scratch.data_ptr(),
+                             scratch.numel(), 0 if marker is None else marker.cuda_event)
         _lib.check(rc, "spd_fwd")
         if out is None:
             out = dict(zip(_lib.OUTPUT_FIELDS, outs))
