@@ -15,6 +15,7 @@
 
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/core/GradMode.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAStream.h>
 
 #include <array>
@@ -288,17 +289,33 @@ PyObject* held_suarez(PyObject*, PyObject* const* a, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
+// A tensor that is no more than its values in memory: not a subclass of torch.Tensor, with no
+// forward-mode tangent, and with no dispatch key that an operation would have to see (a functorch
+// wrapper, a pending negation).
+bool plain(PyObject* v) {
+  if (!THPVariable_CheckExact(v)) return false;
+  const at::Tensor& t = THPVariable_Unpack(v);
+  constexpr c10::DispatchKeySet seen({
+      c10::DispatchKey::Negative, c10::DispatchKey::Conjugate, c10::DispatchKey::ZeroTensor,
+      c10::DispatchKey::Python, c10::DispatchKey::Functionalize, c10::DispatchKey::Batched,
+      c10::DispatchKey::FuncTorchBatched, c10::DispatchKey::FuncTorchGradWrapper});
+  return !t.key_set().has_any(seen) && !t._fw_grad(0).defined();
+}
+
 // The tensor attributes u_wind, v_wind, temperature and specific_humidity of an object (or the items
-// of a list) when they are what the rollout's kernels take: contiguous float32 on one CUDA device,
-// of one shape, with no gradient to record; false otherwise.
+// of a list) when they are what the rollout's kernels take: plain contiguous float32 on one CUDA
+// device, of one shape, with no gradient to record; false otherwise, and wherever a dispatch mode
+// watches the operations.
 bool planes(PyObject* obj, std::array<at::Tensor, 4>& t) {
+  if (c10::impl::TorchDispatchModeTLS::any_modes_set()) return false;
+  if (PyList_Check(obj) && PyList_GET_SIZE(obj) != 4) return false;
   for (int i = 0; i < 4; ++i) {
-    if (PyList_Check(obj)) {
-      if (PyList_GET_SIZE(obj) != 4 || !THPVariable_Check(PyList_GET_ITEM(obj, i))) return false;
-      t[i] = THPVariable_Unpack(PyList_GET_ITEM(obj, i));
-    } else {
-      t[i] = attribute(obj, g_inputs[i].str);
-    }
+    const auto v = pybind11::reinterpret_steal<pybind11::object>(
+        PyList_Check(obj) ? Py_NewRef(PyList_GET_ITEM(obj, i))
+                          : PyObject_GetAttr(obj, g_inputs[i].str));
+    if (!v) throw python_error();
+    if (!plain(v.ptr())) return false;
+    t[i] = THPVariable_Unpack(v.ptr());
     if (!t[i].is_cuda() || t[i].scalar_type() != at::kFloat || !t[i].is_contiguous() ||
         t[i].dim() < 1 || t[i].numel() == 0 || t[i].device() != t[0].device() ||
         t[i].sizes() != t[0].sizes() || (t[i].requires_grad() && c10::GradMode::is_enabled()))
