@@ -219,8 +219,8 @@ def calls():
         import importlib.machinery
         import importlib.util
 
-        import torch
-        path = os.path.join(HERE, "_calls.torch" + torch.__version__.split("+")[0] + ".so")
+        from .build import calls_path
+        path = calls_path()
         if not os.path.exists(path):
             raise SpeedyLibraryError(
                 f"{path} is missing: build it with `python -c 'import __graft_entry__ as g; "

@@ -3,13 +3,15 @@
 Each translation unit is compiled to an object in parallel, then linked into one shared
 library; objects go to ``jax-gcm_b200/_build/`` (not committed).  Beside it, g++ builds the
 extension module through which the Python calls hand torch tensors to the library
-(``csrc/torch_calls.cpp``), against the installed torch and named by its version.
+(``csrc/torch_calls.cpp``), against the installed torch and named by its version and the
+interpreter's.  The library alone needs no torch.
 """
 from __future__ import annotations
 
 import os
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
@@ -62,14 +64,15 @@ def compile_command(src, verbose=False):
 
 
 def calls_path():
+    """The torch extension module, named by torch's version with its CUDA variant and by the
+    interpreter: what it was built against and for."""
     import torch
-    return os.path.join(HERE, "_calls.torch" + torch.__version__.split("+")[0] + ".so")
+    return os.path.join(HERE, "_calls.torch" + torch.__version__
+                        + sysconfig.get_config_var("EXT_SUFFIX"))
 
 
 def calls_command():
     """The compile command of the torch extension module."""
-    import sysconfig
-
     import torch
     lib = os.path.join(os.path.dirname(torch.__file__), "lib")
     inc = os.path.join(os.path.dirname(torch.__file__), "include")
@@ -103,13 +106,26 @@ def needs_build():
 
 
 def build(force=False, verbose=False):
-    if force or needs_calls():
+    """Builds what is out of date: the library, which needs nvcc alone, then the extension module,
+    where there is a torch with CUDA to build it for.  Returns the library's path."""
+    if force or needs_build():
+        build_library(verbose)
+    try:
+        import torch
+    except ImportError:
+        torch = None
+    if torch is None or torch.version.cuda is None:
+        sys.stderr.write("no torch with CUDA here: the library is built, its torch calls are not\n")
+    elif force or needs_calls():
         res = subprocess.run(calls_command(), capture_output=True, text=True)
         if res.returncode != 0:
             sys.stderr.write(res.stdout + res.stderr)
-            raise RuntimeError("g++ failed: " + " ".join(calls_command()))
-    if not force and not needs_build():
-        return OUT
+            raise RuntimeError("the library is built, the torch extension module is not; g++ failed: "
+                               + " ".join(calls_command()))
+    return OUT
+
+
+def build_library(verbose=False):
     os.makedirs(OBJ_DIR, exist_ok=True)
     jobs = [compile_command(s, verbose) for s in SOURCES]
 
@@ -130,7 +146,6 @@ def build(force=False, verbose=False):
     if res.returncode != 0:
         sys.stderr.write(res.stdout + res.stderr)
         raise RuntimeError("nvcc link failed: " + " ".join(link))
-    return OUT
 
 
 if __name__ == "__main__":
