@@ -212,8 +212,8 @@ _calls = None
 
 def calls():
     """The extension module that hands torch tensors to the library (``csrc/torch_calls.cpp``,
-    built by ``build.py`` for the installed torch).  Raises SpeedyLibraryError when it is
-    missing."""
+    built by ``build.py`` for the installed torch); where that has not been built or does not load,
+    with a warning, the same calls through ctypes, which need the library alone."""
     global _calls
     if _calls is None:
         import importlib.machinery
@@ -221,20 +221,24 @@ def calls():
 
         from .build import calls_path
         path = calls_path()
-        if not os.path.exists(path):
-            raise SpeedyLibraryError(
-                f"{path} is missing: build it with `python -c 'import __graft_entry__ as g; "
-                "g.build()'`")
         lib = load()
         with _lock:
             if _calls is None:
-                loader = importlib.machinery.ExtensionFileLoader("_calls", path)
-                mod = importlib.util.module_from_spec(
-                    importlib.util.spec_from_loader("_calls", loader))
-                loader.exec_module(mod)
-                mod.bind(*(C.cast(f, C.c_void_p).value
-                           for f in (lib.spd_fwd_marked, lib.spd_vjp, lib.spd_held_suarez,
-                                     lib.spd_rollout_step, lib.spd_rollout_reverse)))
+                try:
+                    loader = importlib.machinery.ExtensionFileLoader("_calls", path)
+                    mod = importlib.util.module_from_spec(
+                        importlib.util.spec_from_loader("_calls", loader))
+                    loader.exec_module(mod)
+                    mod.bind(*(C.cast(f, C.c_void_p).value
+                               for f in (lib.spd_fwd_marked, lib.spd_vjp, lib.spd_held_suarez,
+                                         lib.spd_rollout_step, lib.spd_rollout_reverse)))
+                except ImportError as e:
+                    import warnings
+
+                    from . import ctypes_calls as mod
+                    warnings.warn(f"calls go through ctypes, {path} does not load ({e}): build it "
+                                  "with `python -c 'import __graft_entry__ as g; g.build()'`",
+                                  RuntimeWarning, stacklevel=3)
                 _calls = mod
     return _calls
 

@@ -1,4 +1,4 @@
-"""The native calls refuse a field that holds fewer values than the geometry has, before anything
+"""The native calls, and the same through ctypes, refuse a field that holds fewer values than the geometry has, before anything
 reaches the library (nothing is launched: every tensor here is on the host, and the last check, for
 the device, refuses them too)."""
 import ctypes as C
@@ -16,9 +16,11 @@ SURFACE = ("alb0", "sice_am", "snowc_am", "soilw_am", "stl_am", "sea_surface_tem
 TENDENCY = STATE[:4]
 
 
-@pytest.fixture(scope="module")
-def calls():
-    return L.calls()
+@pytest.fixture(scope="module", params=["native", "ctypes"])
+def calls(request):
+    if request.param == "native":
+        return L.calls()
+    return importlib.import_module("jax-gcm_b200.ctypes_calls")
 
 
 def objects():
