@@ -5,8 +5,8 @@
 // member's level set S and per-latitude solar table: neither carries a derivative).  Launch 3
 // runs one thread per column, one block per tile: the reverse pass of speedy_vjp_smem.cuh
 // recomputes the column's forward and walks its terms backwards, writing the state gradients;
-// the 12 parameter gradients are summed per thread, then per warp, then added to the tile's
-// member with one coalesced atomic.  A single instance is one member given by value to the same
+// the 12 parameter gradients are summed per thread, then per warp, then per block, and added to the
+// tile's member with one coalesced atomic.  A single instance is one member given by value to the same
 // kernels.
 //
 // Measured (the whole call, against the fully unrolled reverse pass with its arrays in registers
@@ -33,11 +33,21 @@ namespace spd {
 int check_instance(const spd_desc_t* d, const spd_inputs_t* in, const spd_outputs_t* out);
 Consts make_consts(const spd_desc_t* d, const spd_vgrid_t* vg, const spd_params_t* p);
 
-// Adds the warp's sums of pacc to params, one coalesced atomic.  Sixteen lanes' worth of sums
-// (12 used) are folded by halves: a lane keeps the half of the values its bit selects and adds the
-// other lane's, 16 shuffles where a butterfly per value takes 60.  Every lane must call it.
-__device__ __forceinline__ void warp_add_params(const float* pacc, float* params) {
-  const int lane = threadIdx.x & 31;
+// A block's parameter sums, by warp, and how many of its warps have left theirs.
+struct BlockSums {
+  float warp[kNT / 32][SPD_NUM_DIFF_PARAMS];
+  unsigned arrived;
+};
+
+// Adds the block's sums of pacc to params, one coalesced atomic per tile.  Sixteen lanes' worth of
+// sums (12 used) are folded by halves: a lane keeps the half of the values its bit selects and adds
+// the other lane's, 16 shuffles where a butterfly per value takes 60.  The warps leave their sums in
+// shared memory and the last to come adds them in the warps' order, so that no warp waits and the
+// sums of an instance of one tile are the same on every call (an atomic per warp gave other bits in
+// two of five calls beside another stream's work).  Every thread must call it; the block's barrier
+// before its next tile keeps the tiles apart.
+__device__ __forceinline__ void block_add_params(const float* pacc, float* params, BlockSums& s) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   float v[16];
 #pragma unroll
   for (int j = 0; j < 16; ++j) v[j] = j < SPD_NUM_DIFF_PARAMS ? pacc[j] : 0.0f;
@@ -52,7 +62,22 @@ __device__ __forceinline__ void warp_add_params(const float* pacc, float* params
   }
   v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
   const int j = lane >> 1;
-  if ((lane & 1) == 0 && j < SPD_NUM_DIFF_PARAMS) atomicAdd(params + j, v[0]);
+  if ((lane & 1) == 0 && j < SPD_NUM_DIFF_PARAMS) s.warp[warp][j] = v[0];
+  __threadfence_block();
+  __syncwarp();
+  unsigned before = 0;
+  if (lane == 0) before = atomicAdd(&s.arrived, 1u);
+  before = __shfl_sync(0xffffffffu, before, 0);
+  if (before != kNT / 32 - 1) return;
+  __threadfence_block();
+  if (lane < SPD_NUM_DIFF_PARAMS) {
+    const volatile float(*sums)[SPD_NUM_DIFF_PARAMS] = s.warp;
+    float sum = sums[0][lane];
+#pragma unroll
+    for (int w = 1; w < kNT / 32; ++w) sum += sums[w][lane];
+    atomicAdd(params + lane, sum);
+  }
+  if (lane == 0) s.arrived = 0;
 }
 
 // Start of a call: every member's level set and parameter gradients at zero.  One block.
@@ -122,6 +147,8 @@ __global__ void __launch_bounds__(kNT, kWarpsPerSm / (kNT / 32))
                      int ntiles) {
   extern __shared__ float sm[];
   __shared__ VjpMemberDev m;
+  __shared__ BlockSums sums;
+  if (threadIdx.x == 0) sums.arrived = 0;  // before the first tile's barrier
   constexpr int kWords = sizeof(VjpMemberDev) / sizeof(uint64_t);
   static_assert(kWords <= kNT && sizeof(VjpMemberDev) % sizeof(uint64_t) == 0, "one copy per thread");
   for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
@@ -147,7 +174,7 @@ __global__ void __launch_bounds__(kNT, kWarpsPerSm / (kNT / 32))
     }
 #pragma unroll
     for (int j = 0; j < SPD_NUM_DIFF_PARAMS; ++j) pacc[j] = valid ? pacc[j] : 0.0f;
-    warp_add_params(pacc, load_field(m.gr.params));
+    block_add_params(pacc, load_field(m.gr.params), sums);
   }
 }
 
