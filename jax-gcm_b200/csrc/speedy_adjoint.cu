@@ -1,5 +1,6 @@
 // speedy_adjoint.cu -- the adjoint of the forward: one instance (spd_vjp) or a ragged ensemble
-// of them (spd_ensemble_vjp), both through the same three launches (the first clears what they add to).
+// of them (spd_ensemble_vjp), both through the same three launches (the first clears what the
+// others add to).
 //
 // Launch 2 is the forward's cloud-top pre-pass over the tile list of speedy_ensemble.cuh (each
 // member's level set S and per-latitude solar table: neither carries a derivative).  Launch 3
@@ -10,8 +11,8 @@
 // kernels.
 //
 // Measured (the whole call, against the fully unrolled reverse pass with its arrays in registers
-// and local memory that this replaces): T425 with 16 levels 3,191 -> 942 us, T170 with 16
-// levels and verify 578 -> 213 us, T85 with 16 levels 129 -> 57 us.
+// and local memory that this replaces): T425 with 16 levels 3,195 -> 893 us, T170 with 16
+// levels and verify 578 -> 204 us, T85 with 16 levels 131 -> 51.6 us.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -33,20 +34,17 @@ namespace spd {
 int check_instance(const spd_desc_t* d, const spd_inputs_t* in, const spd_outputs_t* out);
 Consts make_consts(const spd_desc_t* d, const spd_vgrid_t* vg, const spd_params_t* p);
 
-// A block's parameter sums, by warp, and how many of its warps have left theirs.
-struct BlockSums {
-  float warp[kNT / 32][SPD_NUM_DIFF_PARAMS];
-  unsigned arrived;
-};
-
 // Adds the block's sums of pacc to params, one coalesced atomic per tile.  Sixteen lanes' worth of
 // sums (12 used) are folded by halves: a lane keeps the half of the values its bit selects and adds
-// the other lane's, 16 shuffles where a butterfly per value takes 60.  The warps leave their sums in
-// shared memory and the last to come adds them in the warps' order, so that no warp waits and the
-// sums of an instance of one tile are the same on every call (an atomic per warp gave other bits in
-// two of five calls beside another stream's work).  Every thread must call it; the block's barrier
-// before its next tile keeps the tiles apart.
-__device__ __forceinline__ void block_add_params(const float* pacc, float* params, BlockSums& s) {
+// the other lane's, 16 shuffles where a butterfly per value takes 60.  The first warp adds the warps'
+// sums in their order, so that those of an instance of one tile are the same on every call (an atomic
+// per warp gave other bits in two of five calls beside another stream's work).  The warps that wait
+// here hold nothing up: their block's resources are free only when its last warp is done.  (With
+// no barrier, the last warp to come adding the sums, by an atomic count and fences, T85 with 16
+// levels took 52.2 against 50.8 us.)  Every thread must call it; the block's barrier before its
+// next tile keeps the tiles apart.
+__device__ __forceinline__ void block_add_params(const float* pacc, float* params,
+                                                 float (*sums)[SPD_NUM_DIFF_PARAMS]) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   float v[16];
 #pragma unroll
@@ -62,22 +60,14 @@ __device__ __forceinline__ void block_add_params(const float* pacc, float* param
   }
   v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
   const int j = lane >> 1;
-  if ((lane & 1) == 0 && j < SPD_NUM_DIFF_PARAMS) s.warp[warp][j] = v[0];
-  __threadfence_block();
-  __syncwarp();
-  unsigned before = 0;
-  if (lane == 0) before = atomicAdd(&s.arrived, 1u);
-  before = __shfl_sync(0xffffffffu, before, 0);
-  if (before != kNT / 32 - 1) return;
-  __threadfence_block();
-  if (lane < SPD_NUM_DIFF_PARAMS) {
-    const volatile float(*sums)[SPD_NUM_DIFF_PARAMS] = s.warp;
+  if ((lane & 1) == 0 && j < SPD_NUM_DIFF_PARAMS) sums[warp][j] = v[0];
+  __syncthreads();
+  if (threadIdx.x < SPD_NUM_DIFF_PARAMS) {
     float sum = sums[0][lane];
 #pragma unroll
     for (int w = 1; w < kNT / 32; ++w) sum += sums[w][lane];
     atomicAdd(params + lane, sum);
   }
-  if (lane == 0) s.arrived = 0;
 }
 
 // Start of a call: every member's level set and parameter gradients at zero.  One block.
@@ -98,7 +88,7 @@ __global__ void __launch_bounds__(kBlock) vjp_begin(const __grid_constant__ VjpS
 // for it before it adds to a level set.
 template <int KX>
 __device__ __forceinline__ uint32_t prepass_bit(const Consts& K, const spd_inputs_t& in, int c,
-                                                int C, uint32_t* S, ZonalRow* table, int il) {
+                                                int C, ZonalRow* table, int il) {
   if (c < il) table[c] = zonal_row(K.tyear, __ldg(in.sia + c), __ldg(in.coa + c));
   return c < C ? prepass_column<KX>(K, in, c, C) : 0u;
 }
@@ -113,9 +103,9 @@ __global__ void __launch_bounds__(kBlock)
     const int c = tl.col0 + threadIdx.x;
     uint32_t bit;
     switch (m.kx) {  // uniform per block
-      case 16: bit = prepass_bit<16>(K, m.in, c, m.C, m.S, m.table, m.il); break;
-      case 8: bit = prepass_bit<8>(K, m.in, c, m.C, m.S, m.table, m.il); break;
-      default: bit = prepass_bit<7>(K, m.in, c, m.C, m.S, m.table, m.il); break;
+      case 16: bit = prepass_bit<16>(K, m.in, c, m.C, m.table, m.il); break;
+      case 8: bit = prepass_bit<8>(K, m.in, c, m.C, m.table, m.il); break;
+      default: bit = prepass_bit<7>(K, m.in, c, m.C, m.table, m.il); break;
     }
     asm volatile("griddepcontrol.wait;" ::: "memory");
     or_level_set_warp(bit, m.S);
@@ -123,8 +113,10 @@ __global__ void __launch_bounds__(kBlock)
 }
 
 // The adjoint launch: one thread per column (speedy_vjp_smem.cuh), one block per tile with its
-// level arrays in `sm` and no barrier but around its member's record.  The threads past a member's last column run that column again
-// and store nothing, so that every warp is whole (the convection's reverse votes).  Blocks of one
+// level arrays in `sm` and no barrier but around its member's record and its parameter sums.  The threads past a member's
+// last column run that column again and store nothing, so that every warp is whole (the
+// convection's reverse votes).  The times below are of the form that each choice was made on; all
+// of them have come down since (above).  Blocks of one
 // warp, which make room as soon as their columns are done, are no faster: a block's four warps
 // start together and share what they fetch of the code (T425 with 16 levels, 32 / 64 / 128 / 384
 // threads: 1,029 / 972 / 942 / 1,001 us; with 8 levels 563 / 537 / 500 / 515 us).  Barriers at the
@@ -147,10 +139,10 @@ __global__ void __launch_bounds__(kNT, kWarpsPerSm / (kNT / 32))
                      int ntiles) {
   extern __shared__ float sm[];
   __shared__ VjpMemberDev m;
-  __shared__ BlockSums sums;
-  if (threadIdx.x == 0) sums.arrived = 0;  // before the first tile's barrier
+  __shared__ float sums[kNT / 32][SPD_NUM_DIFF_PARAMS];
   constexpr int kWords = sizeof(VjpMemberDev) / sizeof(uint64_t);
-  static_assert(kWords <= kNT && sizeof(VjpMemberDev) % sizeof(uint64_t) == 0, "one copy per thread");
+  static_assert(kWords <= kNT && sizeof(VjpMemberDev) % sizeof(uint64_t) == 0,
+                "one copy per thread");
   for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
     const Tile tl = T.members ? T.tiles[t] : Tile{0, t * kNT};
     __syncthreads();  // the last tile's columns are done with its record
@@ -253,7 +245,8 @@ static int launch_ensemble_vjp(const ClassArgs& A, int kx_layout, bool verify,
   int rc = launch_dependent(ensemble_vjp_prepass, grid_pre, kBlock, 0, st, A, T, ntiles);
   if (rc != SPD_OK) return rc;
   const int warps = grid * (kNT / 32) <= 8 * sms ? kWarps8 : kx_layout > 8 ? kWarps12 : kWarps16;
-  rc = launch_dependent(kAdjoint[2 * warps + verify], grid, kNT, vjp_arena_bytes(kx_layout), st, A, T, ntiles);
+  rc = launch_dependent(kAdjoint[2 * warps + verify], grid, kNT, vjp_arena_bytes(kx_layout), st, A,
+                        T, ntiles);
   if (rc != SPD_OK) return rc;
   return cudaGetLastError() == cudaSuccess ? SPD_OK : SPD_ERR_CUDA;
 }
@@ -312,7 +305,8 @@ int spd_vjp(const spd_desc_t* desc, const spd_vgrid_t* vgrid, const spd_params_t
   T.single.S = reinterpret_cast<uint32_t*>(base + L.levelset);
   T.single.table = reinterpret_cast<ZonalRow*>(base + L.tables);
   T.nmembers = 1;
-  return launch_ensemble_vjp(A, desc->kx, (desc->flags & SPD_FUSE_VERIFY) != 0, T, L.ntiles, 0, st);
+  return launch_ensemble_vjp(A, desc->kx, (desc->flags & SPD_FUSE_VERIFY) != 0, T, L.ntiles, 0,
+                             st);
 }
 
 size_t spd_ensemble_vjp_plan_bytes(const spd_vjp_member_t* members, int nmembers) {
