@@ -38,8 +38,7 @@ class HeldSuarezPhysics(Physics):
         d.sigma_b, d.kf, d.ka, d.ks = self.sigma_b, self.kf, self.ka, self.ks
         d.min_t, d.max_t, d.dt_y, d.dthz, d.kappa = (self.minT, self.maxT, self.dTy, self.dThz,
                                                      self.kappa)
-        for k in range(kx):
-            d.sigma[k] = float(np.float32(geometry.fsg[k]))
+        d.sigma[:kx] = np.asarray(geometry.fsg[:kx], np.float32).tolist()
         return d
 
     def _lat_table(self, geometry: Geometry, device):

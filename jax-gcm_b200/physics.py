@@ -428,11 +428,9 @@ def physics_data_from_diagnostics(d):
     )
 
 
-def current_raw_stream(device_index):
-    """The current CUDA stream of a device as a raw handle (torch's own fast path where it has
-    one; torch.cuda.current_stream otherwise)."""
-    f = getattr(torch._C, "_cuda_getCurrentRawStream", None)
-    return f(device_index) if f is not None else torch.cuda.current_stream(device_index).cuda_stream
+# The current CUDA stream of a device index as a raw handle (torch's own fast path where it has one).
+current_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (
+    lambda device_index: torch.cuda.current_stream(device_index).cuda_stream)
 
 
 class SpeedyPhysics(Physics):
@@ -491,14 +489,15 @@ class SpeedyPhysics(Physics):
                          float(dt), float(self.q_tend_scale))
 
     def _scratch_for(self, desc, device):
-        lib = _lib.load()
-        n = lib.spd_fwd_scratch_bytes(C.byref(desc))
         # The launches of two calls on one scratch must not interleave.  None is dropped while the
         # object lives: a captured graph may hold its address.
-        key = (device, n, current_raw_stream(device.index), get_ident())
+        key = (device.index, current_raw_stream(device.index), get_ident())
         buf = self._scratch.get(key)
         if buf is None:
-            buf = self._scratch[key] = torch.empty(n, dtype=torch.uint8, device=device)
+            n = _lib.load().spd_fwd_scratch_bytes(C.byref(desc))  # the same for every shape, or 0
+            buf = torch.empty(n, dtype=torch.uint8, device=device)
+            if n:
+                self._scratch[key] = buf
         return buf
 
     def compute_tendencies(self, state: PhysicsState, forcing: ForcingData, geometry: Geometry,
@@ -506,10 +505,10 @@ class SpeedyPhysics(Physics):
                            accumulate: bool = False):
         """Tendencies and PhysicsData for ``state``.  ``out`` may give preallocated output
         tensors (they must not overlap the inputs); ``marker`` (a torch.cuda.Event) is recorded
-        between the call's two launches, for timing them separately: after the fused launch
-        (before the fixup) when speculating, after the level-set launch (before the fused one)
-        otherwise (``speculating(accumulate)`` says which).  ``accumulate=True`` adds precnv, precls and the float
-        diagnostics to what ``out`` holds instead of overwriting them (the running sums of
+        beside the call's fused launch, for timing that apart: after it (before the fixup) when
+        speculating, before it (after the level-set launch) otherwise
+        (``speculating(accumulate)`` says which).  ``accumulate=True`` adds precnv, precls and the
+        float diagnostics to what ``out`` holds instead of overwriting them (the running sums of
         DiagnosticsCollector, jcm/model.py:46-64; scale by 1/steps once at the end)."""
         if accumulate and out is None:
             raise ValueError("accumulate=True adds into `out`: pass the running sums")

@@ -21,6 +21,7 @@ def scratch(monkeypatch):
         monkeypatch.setattr(physics, "current_raw_stream", lambda index: stream)
         return phys._scratch_for(desc, torch.device("cpu"))
 
+    monkeypatch.setattr(physics, "current_raw_stream", lambda index: 0)
     on.physics = phys
     return on
 
@@ -37,3 +38,11 @@ def test_threads_do_not_share(scratch):
     t.start()
     t.join()
     assert other[0].data_ptr() != mine.data_ptr() and scratch(11) is mine
+
+
+def test_no_scratch_is_kept_for_an_empty_grid(scratch):
+    from types import SimpleNamespace
+    desc = scratch.physics.desc(SimpleNamespace(nodal_shape=(8, 4, 0)), SimpleNamespace(
+        dt_seconds=1.0, tyear=0.0, model_year=1950, model_step=0), True)
+    assert scratch.physics._scratch_for(desc, torch.device("cpu")).numel() == 0
+    assert scratch(0).numel() > 0
