@@ -91,3 +91,32 @@ def test_forwards_of_one_object_from_two_threads(pkg):
         assert len(got[i]) == 50
         for g in got[i]:
             assert all(torch.equal(a, b) for a, b in zip(g, want[i])), i
+
+
+@pytest.mark.parametrize("warm", [False, True])
+def test_captured_calls(pkg, warm):
+    """A forward and a VJP captured on the graph's own stream, without and with calls before it on
+    another, while the object goes on being called; two graphs of one object."""
+    import torch
+    cases = instances(pkg)
+    phys = pkg.SpeedyPhysics(diagnostics=False)
+    if warm:
+        phys.compute_tendencies(*cases[0][:4])
+    pkg._lib.preload(0)
+    want = [([getattr(pkg.SpeedyPhysics(speculate=False).compute_tendencies(*c[:4])[0], n)
+              for n in STATE[:4]], pkg.adjoint.vjp(phys, *c)[0]) for c in cases]
+    torch.cuda.synchronize()
+    graphs = []
+    for c in cases:
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            tend, _ = phys.compute_tendencies(*c[:4])
+            grad, _ = pkg.adjoint.vjp(phys, *c)
+        graphs.append((g, tend, grad))
+    for i in range(6):
+        (g, tend, grad), (wt, wg) = graphs[i % 2], want[i % 2]
+        g.replay()
+        phys.compute_tendencies(*cases[1 - i % 2][:4])
+        torch.cuda.synchronize()
+        assert all(torch.equal(getattr(tend, n), w) for n, w in zip(STATE[:4], wt)), i
+        assert all(torch.equal(getattr(grad, n), getattr(wg, n)) for n in STATE), i
