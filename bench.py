@@ -38,7 +38,7 @@ sys.path.insert(0, ROOT)
 NCU_TRAFFIC_PER_COLUMN = {"ensemble": (96.185856e6 + 54.689792e6) / 466944,
                           "t425": (196.726784e6 + 168.578816e6) / 819200}
 NCU_WARP_INSTRUCTIONS = {"ensemble": 101748554.0, "t425": 212669550.0,
-                         "adjoint_t170": 76210642.0}
+                         "adjoint_t170": 76158872.0}
 
 
 def parse_args():

@@ -158,8 +158,10 @@ size_t spd_fwd_scratch_bytes(const spd_desc_t* desc);
  * column whole in one pass (all terms, verify_tendencies when on, every output); then a fixup that
  * returns at once when the prediction held.  Under SPD_NO_SPECULATION a light launch over every
  * column forms the level set first instead, and there is no fixup.  They are the batched kernels
- * below run on a one-member plan, so the results equal the batched path's bitwise.  `scratch` must be 256-byte aligned and at least spd_fwd_scratch_bytes(desc) long;
- * it is initialised by the call. */
+ * below run on a one-member plan, so the results equal the batched path's bitwise.  `scratch` must
+ * be 256-byte aligned and at least spd_fwd_scratch_bytes(desc) long.  It needs no initialisation:
+ * of what it holds the call uses one word, as its prediction, and checks that; a scratch that the
+ * instance's last call used makes the prediction hold. */
 int spd_fwd(const spd_desc_t* desc, const spd_vgrid_t* vgrid, const spd_params_t* params,
             const spd_inputs_t* in, const spd_outputs_t* out, void* scratch,
             size_t scratch_bytes, void* stream);

@@ -132,9 +132,9 @@ class Ensemble:
         return tuple(sorted((m.geometry.nodal_shape for m in self.members)))
 
     def forward(self, grid_blocks=None, marker=None):
-        """Runs every member.  ``marker`` (a torch.cuda.Event) is recorded between the two
-        launches, for timing them separately: after the fused launch (before the fixup) when
-        ``speculate``, after the level-set launch (before the fused one) otherwise.  With
+        """Runs every member.  ``marker`` (a torch.cuda.Event) is recorded beside the fused
+        launch, for timing that apart: after it (before the fixup) when ``speculate``, before it
+        (after the level-set launch) otherwise.  With
         ``speculate`` each member's cloud-top level set is predicted from the previous call
         (the plan keeps it), checked on the device, and only members whose prediction missed
         are computed again (``redone()`` counts them)."""

@@ -41,9 +41,9 @@ FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC"]
 # keep their distances at the printed digits; the only values flushed are transmissivities below
 # 1e-38).  The adjoint keeps subnormals and is compiled without contraction too: the values that
 # decide its branches are rounded like the reference's (its division is fdiv in
-# csrc/speedy_vjp.h, which rounds like the IEEE one), its fused multiply-adds are written out, and
-# its two register budgets give the same bits, so that a member's gradients do not depend on the
-# batch it is served in.
+# csrc/speedy_vjp.h, which rounds like the IEEE one away from the ends of the exponent range), its
+# fused multiply-adds are written out, and its three register budgets, with and without verify,
+# give the same bits, so that a member's gradients do not depend on the batch it is served in.
 FORWARD_FLAGS = ["-fmad=false", "-prec-div=false", "-ftz=true"]
 SOURCE_FLAGS = {"csrc/speedy_ensemble.cu": FORWARD_FLAGS,
                 "csrc/speedy_selftest.cu": FORWARD_FLAGS,  # checks the forward's arithmetic

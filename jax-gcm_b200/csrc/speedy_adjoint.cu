@@ -11,8 +11,8 @@
 // kernels.
 //
 // Measured (the whole call, against the fully unrolled reverse pass with its arrays in registers
-// and local memory that this replaces): T425 with 16 levels 3,195 -> 893 us, T170 with 16
-// levels and verify 578 -> 204 us, T85 with 16 levels 131 -> 51.6 us.
+// and local memory that this replaces): T425 with 16 levels 3,195 -> 890 us, T170 with 16
+// levels and verify 578 -> 204 us, T85 with 16 levels 131 -> 51 us.
 #include <cuda_runtime.h>
 #include <stdint.h>
 

@@ -70,10 +70,10 @@ __device__ __forceinline__ void prefetch_tile_rows(int nrows, RowFn row) {
 // member's predicted level set P and a fixup launch redoes the members whose prediction missed;
 // otherwise a level-set launch forms every T before the fused launch reads it.  grid_blocks:
 // > 0 = the fused launch's persistent grid; 0 or SPD_GRID_PER_TILE = one block per tile (the
-// 61-member ensemble takes 150 us so, 161 us as a persistent grid of SMs x resident blocks,
-// whose blocks own unequal strides of 8- and 16-level tiles).  verify: whether any class fuses
-// verify.  kx_layout is the largest level count among the
-// tiles (it sizes the fused launch's shared-memory arena).
+// 61-member ensemble took 143 us so, 161 us as a persistent grid of SMs x resident blocks, whose
+// blocks own unequal strides of 8- and 16-level tiles).  verify: whether any class fuses verify.
+// kx_layout is the largest level count among the tiles (it sizes the fused launch's shared-memory
+// arena).
 int launch_forward(const ClassArgs& A, const TileSource& T, int ntiles, int kx_layout,
                    int grid_blocks, bool speculate, bool verify, cudaStream_t st,
                    cudaEvent_t marker);

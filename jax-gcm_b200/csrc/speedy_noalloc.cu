@@ -4,10 +4,10 @@
 // ctypes stub) that only forwards the state, forcing and tendency buffers handed to it, or a
 // process whose device memory is owned entirely by another runtime's pooling allocator.  This
 // entry point needs no scratch argument and performs no allocation: its scratch lives in the
-// fixed file-scope device array below.  The instance's level-set state takes its first 256 bytes; the rest holds up to SPD_NOALLOC_MAX_IL rows of a
-// per-latitude table (the size limit of the entry point; the present kernels form each
-// column's solar row themselves and leave it unused).  Every GPU that loads the library keeps
-// that array (65,792 bytes) until the process exits.
+// fixed file-scope device array below.  The instance's level-set state takes its first 256 bytes;
+// the rest holds up to SPD_NOALLOC_MAX_IL rows of a per-latitude table (the size limit of the entry
+// point; the present kernels form each column's solar row themselves and leave it unused).  Every
+// GPU that loads the library keeps that array (65,792 bytes) until the process exits.
 #include <cuda_runtime.h>
 #include <stdint.h>
 

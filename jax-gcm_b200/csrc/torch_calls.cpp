@@ -1,14 +1,15 @@
 // torch_calls.cpp -- the plain calls on torch tensors: gathers the field pointers, allocates the
 // results and calls the C ABI, for physics.py, adjoint.py, held_suarez.py and rollout.py.
 //
-// A small call is bound by the host: through ctypes a T21 call with its diagnostics took 91 us, of
-// which the device works 17 (21 torch.empty calls of 2.4 us each, 38 pointers, the structures).
-// Through this module it takes 38 us (T85 with 16 levels 45 -> 25, a T42 VJP with 8 levels 44 ->
-// 31, a 361 x 181 Held-Suarez call 27 -> 16); 21 of the 38 are the 21 result tensors.  It does the
-// same in one call: 17 attribute reads and checks, one allocation per result
-// through torch's allocator, and the library call with the interpreter's lock released.  Nothing is
-// kept between calls.  The library's entry points come in as addresses (bind), so that this module
-// does not depend on which build of the library is loaded.
+// A small call is bound by the host: through ctypes (ctypes_calls.py, the same calls for a torch that
+// this module has not been built for) a T21 call with its diagnostics took 91 us, of which the
+// device works 17 (21 torch.empty calls of 2.4 us each, 38 pointers, the structures).  Through this
+// module it takes 37 us (T85 with 16 levels 45 -> 24, a 361 x 181 Held-Suarez call 27 -> 16; a T42
+// VJP with 8 levels 44 -> 28.7, which the device bounds); 21 of the 37 are the 21 result tensors.
+// It does the same in one call: 17 attribute reads and checks, one allocation per result through
+// torch's allocator, and the library call with the interpreter's lock released.  Nothing is kept
+// between calls.  The library's entry points come in as addresses (bind), so that this module does
+// not depend on which build of the library is loaded.
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/utils/pybind.h>
